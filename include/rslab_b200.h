@@ -291,11 +291,10 @@ int rslab_solve_profile(rslab_fac_handle* fac, int64_t nrhs, double* kind_ms, in
  * 5 forward push, 6 backward dots, 7 backward diagonal, 8-11 see below, 13
  * multifrontal extend-add, 14 G = L21 D, 15 diagonal-block inverses, 17
  * tensor-core panel Schur (tcgen05 or DMMA tiles), 18/19 forward/backward
- * block-chain solve, 21 deep rows as a product with the block transform, 22
- * block transform, 23 forward push partial-sum reduction, 24 multifrontal
- * contribution block, -1 other; 12, 16 and 20 are not launched any more: the
- * chain items gather their own right-hand sides and sum split dots), grid
- * size and device ms.  *count = rows available; at most cap are written.
+ * block-chain solve, 23 forward push partial-sum reduction, 24 multifrontal
+ * contribution block, -1 other; 12, 16, 20, 21 and 22 are not launched any
+ * more: the chain items gather their own right-hand sides and sum split dots,
+ * and the deep rows need no block transform), grid size and device ms.  *count = rows available; at most cap are written.
  * A measurement aid with no reference counterpart.  Kinds 8-11 are the
  * tensor-core cmod's GEMM tiles, its assembly and the real / complex operand
  * split. */

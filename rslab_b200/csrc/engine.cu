@@ -22,6 +22,7 @@
 
 #include "../../include/rslab_b200.h"
 #include "device/factor_kernels.cuh"
+#include "device/panel.cuh"
 #include "device/cmod_tc.cuh"
 #include "device/cmod_mm.cuh"
 #include "device/solve_kernels.cuh"
@@ -123,14 +124,13 @@ struct Launch {
   int kind;
   long long task_off;  // into the int4 / int2 / int task arrays
   int ntasks;
-  int nb_slot;         // getf2/deep: scratch stride nb; chain solves: ticket counter
+  int nb_slot;         // getf2/deep: widest block of the launch; chain solves: ticket counter
   int side = 0;        // factor: 1 = may run on the side stream, overlapping the next block's
                        // getf2 / deep-row launches (Schur update beyond the next block);
                        // 2 = on the cmod stream, overlapping the whole level (early
                        // tensor-core cmod of the next level, tagged by nb_slot)
-  int narrow = 0;      // getf2: 0, or the block width that sizes the shared memory of a
-                       // launch of narrow tasks (the 128-thread kernel); chain solves: 1 =
-                       // one chain per block over every column of the pass
+  int narrow = 0;      // front cb: 1 = DMMA tiles; chain solves: 1 = one chain per block over
+                       // every column of the pass
 };
 
 }  // namespace
@@ -204,8 +204,6 @@ struct rslab_sym_handle {
   std::vector<int> pull_ptr, pull_src;
   std::vector<int2> dots_red;  // per supernode: (first slot, chunks) of its split backward dots
   std::vector<Launch> fplan, fwdplan, bwdplan;
-  int max_getf2_tasks = 0;
-  int max_nb = 64;
   double flops_model = 0, flops_proxy = 0;
   // algorithmic real-field flops (multiply + add = 2) per launch kind:
   // [0] assembly, [1] cmod, [2] getf2, [3] deep-row replay, [4] panel Schur
@@ -644,7 +642,6 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
 
   // Launch plan.
   const int nb_small = H.panel_nb, nb_big = std::max(H.panel_nb, 128);
-  H.max_nb = nb_big;
   auto nb_of = [&](int s) { return S.sn[s].ncol >= 512 ? nb_big : nb_small; };
   std::vector<std::vector<Launch>> bw_levels;
   std::vector<int> lv_of(ns, 0);
@@ -725,25 +722,22 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
     for (int64_t s : lvl) maxblocks = std::max(maxblocks, (int)((S.sn[s].ncol + nb_of(s) - 1) / nb_of(s)));
     for (int b = 0; b < maxblocks; ++b) {
       Launch G{L_GETF2, (long long)H.t4.size(), 0, 0};
-      std::vector<int4> deep, make_m, deep_mm, schur, schur_tc, schur_r, schur_tc_r, narrow;
-      int slot = 0, launch_nb = 0, narrow_nb = 0;
+      std::vector<int4> deep, schur, schur_tc, schur_r, schur_tc_r, narrow;
+      int max_pw = 0, max_narrow = 0, max_deep = 0;
+      bool any = false;
       for (int64_t s : lvl) {
         int nb = nb_of(s), nc = (int)S.sn[s].ncol, nr = H.nrow[s];
         int kb = b * nb;
         if (kb >= nc) continue;
+        any = true;
         int ke = std::min(kb + nb, nc);
         bool fuse = (nr - ke) <= FUSE_DEEP_ROWS;
-        // narrow blocks with few deep rows (most leaves of a 3D problem are
-        // one to a few columns) go to a 128-thread launch: several CTAs per
-        // SM instead of one or two 512-thread ones
-        const bool nar = ke - kb <= GETF2_NARROW_PW && nr - ke <= GETF2_NARROW_DEEP;
-        (nar ? narrow : H.t4).push_back(make_int4((int)s, kb, slot, fuse ? 1 : 0));
-        if (nar) narrow_nb = std::max(narrow_nb, nb);
-        launch_nb = std::max(launch_nb, nb);
+        const bool nar = ke - kb <= GF_NARROW_PW;
+        (nar ? narrow : H.t4).push_back(make_int4((int)s, kb, 0, fuse ? 1 : 0));
+        (nar ? max_narrow : max_pw) = std::max(nar ? max_narrow : max_pw, ke - kb);
         if (!fuse) {
-          for (int r0 = ke; r0 < nr; r0 += DEEP_R) deep.push_back(make_int4((int)s, kb, slot, r0));
-          for (int r0 = ke; r0 < nr; r0 += MM_ROWS) deep_mm.push_back(make_int4((int)s, kb, slot, r0));
-          for (int i0 = 0; i0 < ke - kb; i0 += MM_RB) make_m.push_back(make_int4((int)s, kb, slot, i0));
+          max_deep = std::max(max_deep, ke - kb);
+          for (int r0 = ke; r0 < nr; r0 += DEEP_R) deep.push_back(make_int4((int)s, kb, 0, r0));
         }
         int mt = nr - ke, cw = nc - ke;
         const double pw = ke - kb;
@@ -758,32 +752,25 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
         for (int c0 = 0; c0 < cw; c0 += TC_N)
           for (int r0 = (c0 / TC_M) * TC_M; r0 < mt; r0 += TC_M)
             (c0 < nxt ? schur_tc : schur_tc_r).push_back(make_int4((int)s, kb, r0, c0));
-        ++slot;
+      }
+      if (!any) continue;
+      // narrow blocks ride in the launch of the wider ones (one launch less on
+      // the block chain) unless there are enough of them to fill the GPU with
+      // the small CTAs
+      if (max_pw > 0 && narrow.size() < GF_NARROW_MIN) {
+        H.t4.insert(H.t4.end(), narrow.begin(), narrow.end());
+        narrow.clear();
       }
       G.ntasks = (int)(H.t4.size() - G.task_off);
-      G.nb_slot = launch_nb;
-      if (!slot) continue;
+      G.nb_slot = max_pw;
       if (G.ntasks) H.fplan.push_back(G);
       if (!narrow.empty()) {
-        // the same scratch slots and stride as the wide launch of this block
-        Launch Gn{L_GETF2, (long long)H.t4.size(), (int)narrow.size(), launch_nb};
-        Gn.narrow = narrow_nb;
+        H.fplan.push_back(Launch{L_GETF2, (long long)H.t4.size(), (int)narrow.size(), max_narrow});
         H.t4.insert(H.t4.end(), narrow.begin(), narrow.end());
-        H.fplan.push_back(Gn);
       }
-      H.max_getf2_tasks = std::max(H.max_getf2_tasks, slot);
       if (!deep.empty()) {
-        Launch D{L_DEEP, (long long)H.t4.size(), (int)deep.size(), launch_nb};
+        H.fplan.push_back(Launch{L_DEEP, (long long)H.t4.size(), (int)deep.size(), max_deep});
         H.t4.insert(H.t4.end(), deep.begin(), deep.end());
-        H.fplan.push_back(D);
-        // the same rows as one product with the block transform (tensor-core
-        // engine of the single-precision fields): M, then A21 M
-        Launch Mm{L_MAKE_M, (long long)H.t4.size(), (int)make_m.size(), launch_nb};
-        H.t4.insert(H.t4.end(), make_m.begin(), make_m.end());
-        H.fplan.push_back(Mm);
-        Launch Dm{L_DEEP_MM, (long long)H.t4.size(), (int)deep_mm.size(), launch_nb};
-        H.t4.insert(H.t4.end(), deep_mm.begin(), deep_mm.end());
-        H.fplan.push_back(Dm);
       }
       if (!schur.empty()) {
         Launch C{L_SCHUR, (long long)H.t4.size(), (int)schur.size(), 0};
@@ -961,20 +948,42 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
 // Chunk depth of the tile engine for an element size (KChunk<T>::v).
 size_t kchunk(size_t es) { return es == 16 ? 16 : 32; }
 size_t smem_schur(size_t es) { return 2 * kchunk(es) * TILE * es; }
-// Deep-row staging (DEEP_R + 1) x nb plus the replay program, 16-byte aligned.
-size_t smem_replay(size_t es, int nb) {
-  return (((size_t)(DEEP_R + 1) * nb * es + 15) & ~size_t(15)) + (size_t)nb * (3 * es + 4 + 1) + 16;
-}
-size_t smem_getf2(size_t es, int nb) {
-  size_t a = (size_t)nb * (nb + 1) / 2 * es + 8 * nb * es + 16 + 32 * 8 + 32 * 4 + 16 * 4 + 4 * nb * 4;
-  return std::max(a, smem_replay(es, nb)) + 64;
-}
-size_t smem_deep(size_t es, int nb) { return smem_replay(es, nb) + 64; }
 size_t smem_diag_inv(size_t es) { return (size_t)TB * (TB + 1) * 2 * es; }
 
-// Threads of the BK panel kernel: its per-step trailing update is
-// latency-bound, so 16 warps hide more of it than 8.
-constexpr int GETF2_NT = 512;
+// The panel kernels of a launch whose widest block has `pw` columns: the
+// smallest k_getf2 instance (64 threads up to 32 columns, 256 above) and the
+// smallest k_deep one (8 columns per slot) that hold it.
+template <typename T>
+void launch_getf2(int pw, int ntasks, cudaStream_t st, const FactorArgs& fa, const int4* tasks, int nb_small,
+                  int nb_big) {
+  if (pw <= GF_NARROW_PW)
+    k_getf2<T, GF_NARROW_G, 4><<<ntasks, 64, smem_getf2(sizeof(T), GF_NARROW_PW), st>>>(fa, tasks, nb_small, nb_big);
+  else if (pw <= GF_MID_PW)
+    k_getf2<T, GF_G, 4><<<ntasks, 256, smem_getf2(sizeof(T), GF_MID_PW), st>>>(fa, tasks, nb_small, nb_big);
+  else
+    k_getf2<T, GF_G, 8><<<ntasks, 256, smem_getf2(sizeof(T), GF_WIDE_PW), st>>>(fa, tasks, nb_small, nb_big);
+}
+template <typename T, bool EXACT>
+void launch_deep(int pw, int ntasks, cudaStream_t st, const FactorArgs& fa, const int4* tasks, int nb_small,
+                 int nb_big) {
+  if (pw <= GF_MID_PW)
+    k_deep<T, 8, EXACT><<<ntasks, DEEP_NT, smem_deep(sizeof(T), GF_MID_PW), st>>>(fa, tasks, nb_small, nb_big);
+  else
+    k_deep<T, 16, EXACT><<<ntasks, DEEP_NT, smem_deep(sizeof(T), GF_WIDE_PW), st>>>(fa, tasks, nb_small, nb_big);
+}
+// Their shared-memory limits (once per device).
+template <typename T>
+void panel_attrs() {
+  const size_t es = sizeof(T);
+  constexpr auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  CK(cudaFuncSetAttribute(k_getf2<T, GF_NARROW_G, 4>, A, (int)smem_getf2(es, GF_NARROW_PW)));
+  CK(cudaFuncSetAttribute(k_getf2<T, GF_G, 4>, A, (int)smem_getf2(es, GF_MID_PW)));
+  CK(cudaFuncSetAttribute(k_getf2<T, GF_G, 8>, A, (int)smem_getf2(es, GF_WIDE_PW)));
+  CK(cudaFuncSetAttribute(k_deep<T, 8, true>, A, (int)smem_deep(es, GF_MID_PW)));
+  CK(cudaFuncSetAttribute(k_deep<T, 16, true>, A, (int)smem_deep(es, GF_WIDE_PW)));
+  CK(cudaFuncSetAttribute(k_deep<T, 8, false>, A, (int)smem_deep(es, GF_MID_PW)));
+  CK(cudaFuncSetAttribute(k_deep<T, 16, false>, A, (int)smem_deep(es, GF_WIDE_PW)));
+}
 
 // Fields whose descendant updates can run on the tf32 tensor cores.
 template <typename T> struct TensorCmod { static constexpr bool ok = false; };
@@ -1043,23 +1052,8 @@ struct KernelSetup {
     }
     CK(cudaFuncSetAttribute(k_schur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_schur(es)));
     CK(cudaFuncSetAttribute(k_front_cb<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_schur(es)));
-    CK(cudaFuncSetAttribute(k_getf2<T, GETF2_NT, getf2_wide_minb(sizeof(T))>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem_getf2(es, 128)));
-    CK(cudaFuncSetAttribute(k_getf2<T, 256, getf2_mid_minb(sizeof(T))>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem_getf2(es, 128)));
-    CK(cudaFuncSetAttribute(k_getf2<T, 128, getf2_narrow_minb(sizeof(T))>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_getf2(es, 128)));
-    if constexpr (TensorCmod<T>::ok)
-      CK(cudaFuncSetAttribute(k_getf2_ll<T, GETF2_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem_getf2_ll_bytes<T>(128)));
-    CK(cudaFuncSetAttribute(k_deep<T, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_deep(es, 128)));
+    panel_attrs<T>();
     CK(cudaFuncSetAttribute(k_diag_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diag_inv(es)));
-    CK(cudaFuncSetAttribute(k_deep_mm<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_deep_mm_bytes<T>()));
-    CK(cudaFuncSetAttribute(k_make_m<T, 32 * MM_RB, make_m_sl(sizeof(T))>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem_make_m_bytes(es, 128, make_m_sl(sizeof(T)))));
-    CK(cudaFuncSetAttribute(k_make_m<T, 32 * MM_RB, MAKE_M_SL_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem_make_m_bytes(es, 128, MAKE_M_SL_WIDE)));
     solve_nr_attrs<T, 1>();
     solve_nr_attrs<T, 4>();
     solve_nr_attrs<T, RHS_MAX>();
@@ -1096,8 +1090,6 @@ struct rslab_fac_handle {
   unsigned long long* cnt3 = nullptr;
   double* floor_dev = nullptr;          // force-accept static-pivot floor (device)
   unsigned long long* amax_dev = nullptr;
-  void* scratch = nullptr;
-  long long scratch_stride = 0;
   void* gpool = nullptr;  // G_k = L21_k D_k of every updater (read by both cmod engines)
   void* cbpool = nullptr; // multifrontal variant: every supernode's contribution block
   void* linv = nullptr;   // inverse diagonal blocks of the wide supernodes
@@ -1185,8 +1177,6 @@ FactorArgs make_fargs(rslab_fac_handle& F) {
   a.dsub = F.dsub;
   a.kind = F.kind;
   a.lperm = F.lperm;
-  a.scratch = F.scratch;
-  a.scratch_stride = F.scratch_stride;
   a.status = F.status;
   a.perturb_floor = F.set.on_zero_pivot == RSLAB_PIVOT_PERTURB ? F.set.abs_floor : -1.0;
   a.gpool = F.gpool;
@@ -1259,9 +1249,6 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
   // fields also run their panel Schur / deep rows on the tensor-core kernels
   const bool mm = F.set.schur_engine == RSLAB_SCHUR_TENSOR;
   const bool use_tc = TensorCmod<T>::ok && mm;
-  // deep rows of tall panels as a product with the block transform on the
-  // tensor engine of every field; the FMA engine replays them row by row
-  fa.deep_mm = mm ? 1 : 0;
   // multifrontal variant: contribution blocks and extend-add instead of cmod
   const bool mf = F.set.method == RSLAB_METHOD_MULTIFRONTAL;
   if (mf) CK(cudaMemsetAsync(F.cbpool, 0, (size_t)std::max(H.cb_elems, 1LL) * es, st));
@@ -1286,8 +1273,6 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
       case L_MAKE_G: return !use_tc && !mf;  // G_k of the CUDA-core cmod and of the DMMA tiles
       case L_EXT_ADD: return mf;
       case L_FRONT_CB: return mf && (L.narrow != 0) == (mm && !TensorCmod<T>::ok);  // DMMA tiles or FMA tiles
-      case L_DEEP: return !fa.deep_mm;
-      case L_MAKE_M: case L_DEEP_MM: return fa.deep_mm != 0;
       case L_SCHUR: return !mm;
       case L_SCHUR_TC: return mm;  // tcgen05 tiles (f32 / c32) or DMMA tiles (f64 / c64)
       default: return true;
@@ -1311,8 +1296,7 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
       CK(cudaEventRecord(F.ev_fork, st));
       CK(cudaStreamWaitEvent(F.st2, F.ev_fork, 0));
       ls = F.st2;
-    } else if (side_pending && L.kind != L_GETF2 && L.kind != L_DEEP && L.kind != L_MAKE_M &&
-               L.kind != L_DEEP_MM) {
+    } else if (side_pending && L.kind != L_GETF2 && L.kind != L_DEEP) {
       CK(cudaStreamWaitEvent(st, F.ev_join, 0));
       side_pending = false;
     }
@@ -1361,63 +1345,15 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
                                                                  H.d_poff, (const T*)F.panel, F.status, (T*)F.linv,
                                                                  H.d_linv_off);
         break;
-      case L_GETF2: {
-        FactorArgs f2 = fa;
-        f2.scratch_stride = getf2_scratch_stride(L.nb_slot, (long long)es);
-        if (L.narrow) {  // narrow blocks: the bit-exact form on 4 warps, every field
-          k_getf2<T, 128, getf2_narrow_minb(sizeof(T))>
-              <<<L.ntasks, 128, smem_getf2(es, L.narrow), ls>>>(f2, H.d_t4 + L.task_off, nb_small, nb_big);
-          break;
-        }
-        if constexpr (TensorCmod<T>::ok) {
-          // left-looking form (parity by tolerance, like the rest of the
-          // engine) for launches of a few blocks, where a block's step
-          // latency is the critical path; launches of many blocks take the
-          // right-looking form, which fits two CTAs per SM instead of one
-          if (use_tc && L.ntasks < GETF2_LL_MAX_TASKS) {
-            k_getf2_ll<T, GETF2_NT><<<L.ntasks, GETF2_NT, smem_getf2_ll_bytes<T>(L.nb_slot), ls>>>(
-                f2, H.d_t4 + L.task_off, nb_small, nb_big);
-            break;
-          }
-        }
-        if (L.ntasks >= GETF2_LL_MAX_TASKS)  // many blocks: 8 warps, more CTAs per SM
-          k_getf2<T, 256, getf2_mid_minb(sizeof(T))>
-              <<<L.ntasks, 256, smem_getf2(es, L.nb_slot), ls>>>(f2, H.d_t4 + L.task_off, nb_small, nb_big);
+      case L_GETF2:
+        launch_getf2<T>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
+        break;
+      case L_DEEP:  // the FMA engine in the oracle's operation order, the tensor engine fused
+        if (mm)
+          launch_deep<T, false>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
         else
-          k_getf2<T, GETF2_NT, getf2_wide_minb(sizeof(T))>
-              <<<L.ntasks, GETF2_NT, smem_getf2(es, L.nb_slot), ls>>>(f2, H.d_t4 + L.task_off, nb_small, nb_big);
+          launch_deep<T, true>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
         break;
-      }
-      case L_DEEP: {
-        if (fa.deep_mm) continue;
-        FactorArgs f2 = fa;
-        f2.scratch_stride = getf2_scratch_stride(L.nb_slot, (long long)es);
-        k_deep<T, 256><<<L.ntasks, 256, smem_deep(es, L.nb_slot), ls>>>(f2, H.d_t4 + L.task_off, nb_small, nb_big);
-        break;
-      }
-      case L_MAKE_M: {
-        if (!fa.deep_mm) continue;
-        FactorArgs f2 = fa;
-        f2.scratch_stride = getf2_scratch_stride(L.nb_slot, (long long)es);
-        if (L.ntasks >= GETF2_LL_MAX_TASKS)  // many blocks: smaller slices, more CTAs per SM
-          k_make_m<T, 32 * MM_RB, MAKE_M_SL_WIDE>
-              <<<L.ntasks, 32 * MM_RB, smem_make_m_bytes(es, L.nb_slot, MAKE_M_SL_WIDE), ls>>>(
-                  f2, H.d_t4 + L.task_off, nb_small, nb_big);
-        else
-          k_make_m<T, 32 * MM_RB, make_m_sl(sizeof(T))>
-              <<<L.ntasks, 32 * MM_RB, smem_make_m_bytes(es, L.nb_slot, make_m_sl(sizeof(T))), ls>>>(
-                  f2, H.d_t4 + L.task_off, nb_small, nb_big);
-        break;
-      }
-      case L_DEEP_MM: {
-        if (!fa.deep_mm) continue;
-        {
-          FactorArgs f2 = fa;
-          f2.scratch_stride = getf2_scratch_stride(L.nb_slot, (long long)es);
-          k_deep_mm<T><<<L.ntasks, 256, smem_deep_mm_bytes<T>(), ls>>>(f2, H.d_t4 + L.task_off, nb_small, nb_big);
-        }
-        break;
-      }
       case L_SCHUR:
         if (mm) continue;
         k_schur<T><<<L.ntasks, TPB, smem_schur(es), ls>>>(fa, H.d_t4 + L.task_off, nb_small, nb_big);
@@ -1450,7 +1386,7 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
                   L.kind == L_SPLIT_R || L.kind == L_SPLIT_C || L.kind == L_EXT_ADD || L.kind == L_FRONT_CB) ? 1
                  : (L.kind == L_DIAG_INV || L.kind == L_SCHUR_TC)             ? 4
                  : L.kind == L_GETF2                                           ? 2
-                 : (L.kind == L_DEEP || L.kind == L_DEEP_MM || L.kind == L_MAKE_M) ? 3
+                 : L.kind == L_DEEP                                            ? 3
                                                                                : 4,
                  L.ntasks, L.kind);
     if (ls == F.st3) {
@@ -2369,9 +2305,6 @@ static int factor_impl(rslab_sym_handle* sym, int dtype, int dtype_hi, const voi
     F->cnt3 = F->al<unsigned long long>(3);
     F->aval = F->al<unsigned char>(sym->nnz * es);
     CK(cudaMallocHost(&F->h_status, 4 * sizeof(int)));
-    const long long nbm = sym->max_nb;
-    F->scratch_stride = getf2_scratch_stride(nbm, (long long)es);
-    F->scratch = F->al<unsigned char>((size_t)std::max(1, sym->max_getf2_tasks) * F->scratch_stride);
     F->linv = F->al<unsigned char>((size_t)std::max(sym->linv_elems, 1LL) * es);
     if (F->set.on_zero_pivot == RSLAB_PIVOT_FORCE_ACCEPT) {
       F->floor_dev = F->al<double>(1);
@@ -2865,8 +2798,8 @@ int rslab_metis_order(int64_t n, const int64_t* col_ptr, const int64_t* row_idx,
 // cudaMalloc latency or risk an out-of-memory failure mid-run.  For them
 // rslab_panel_factor_noalloc runs the blocked Bunch-Kaufman panel kernels
 // (getf2, deep-row replay, in-panel Schur) on one caller-owned dense panel
-// with every piece of scratch (the per-block multiplier snapshot, swap log,
-// the panel's structure and the launch task lists) placed in the file-scope
+// with every piece of scratch (the panel's structure and the launch task
+// lists) placed in the file-scope
 // array below instead of memory obtained from an allocator.  The structure
 // and the task lists are written into that array by a small kernel, so no
 // host buffer has to outlive the call.  The array is 1 MiB and, like every
@@ -2878,6 +2811,7 @@ namespace {
 constexpr int64_t NOALLOC_MAX_NROW = 4096;
 constexpr int64_t NOALLOC_MAX_NCOL = 1024;
 constexpr size_t NOALLOC_BYTES = size_t(1) << 20;
+constexpr int NOALLOC_FUSE_ROWS = 192;  // deep rows that a block's getf2 solves itself (fewer task-list entries)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
@@ -2923,7 +2857,7 @@ int noalloc_count(int nrow, int ncol, int nb, std::vector<NoallocSeg>& segs) {
   int t = 0;
   for (int kb = 0; kb < ncol; kb += nb) {
     const int ke = std::min(kb + nb, ncol);
-    const bool fuse = (nrow - ke) <= FUSE_DEEP_ROWS;
+    const bool fuse = (nrow - ke) <= NOALLOC_FUSE_ROWS;
     segs.push_back({L_GETF2, t, 1});
     t += 1;
     if (!fuse) {
@@ -2952,7 +2886,7 @@ __global__ void k_noalloc_plan(NoallocStruct* ns, int4* tasks, int nrow, int nco
   int t = 0;
   for (int kb = 0; kb < ncol; kb += nb) {
     const int ke = min(kb + nb, ncol);
-    const bool fuse = (nrow - ke) <= FUSE_DEEP_ROWS;
+    const bool fuse = (nrow - ke) <= NOALLOC_FUSE_ROWS;
     if (threadIdx.x == 0) tasks[t] = make_int4(0, kb, 0, fuse ? 1 : 0);
     t += 1;
     if (!fuse) {
@@ -2979,8 +2913,7 @@ void noalloc_attrs() {
   std::lock_guard<std::mutex> g(mu);
   if (done[dev]) return;
   const size_t es = sizeof(T);
-  CK(cudaFuncSetAttribute(k_getf2<T, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_getf2(es, 128)));
-  CK(cudaFuncSetAttribute(k_deep<T, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_deep(es, 128)));
+  panel_attrs<T>();
   CK(cudaFuncSetAttribute(k_schur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_schur(es)));
   done[dev] = true;
 }
@@ -2993,8 +2926,10 @@ void noalloc_panel(unsigned char* base, T* panel, int nrow, int ncol, int panel_
   const int nb = ncol >= 512 ? nb_big : nb_small;
   std::vector<NoallocSeg> segs;
   const int ntasks = noalloc_count(nrow, ncol, nb, segs);
-  const size_t snap_bytes = ((size_t)nb_big * nb_big * es + 3 * nb_big * 4 + 255) / 256 * 256;
-  const size_t off_snap = 256, off_tasks = off_snap + snap_bytes;
+  // one block of nb_big columns is kept free ahead of the task lists: the
+  // largest panel accepted is part of the entry point's contract
+  const size_t block_bytes = ((size_t)nb_big * nb_big * es + 3 * nb_big * 4 + 255) / 256 * 256;
+  const size_t off_tasks = 256 + block_bytes;
   const size_t need = off_tasks + (size_t)ntasks * sizeof(int4);
   if (need > NOALLOC_BYTES)
     throw RslabError(Status::InvalidInput, "panel needs " + std::to_string(need) +
@@ -3016,16 +2951,14 @@ void noalloc_panel(unsigned char* base, T* panel, int nrow, int ncol, int panel_
   fa.dsub = dsub;
   fa.kind = kind;
   fa.lperm = lperm;
-  fa.scratch = base + off_snap;
-  fa.scratch_stride = (long long)snap_bytes;
   fa.status = status;
   fa.perturb_floor = -1.0;
   const int4* dt = reinterpret_cast<const int4*>(base + off_tasks);
   for (const NoallocSeg& g : segs) {
     if (g.kind == L_GETF2)
-      k_getf2<T, 256><<<g.cnt, 256, smem_getf2(es, nb), st>>>(fa, dt + g.off, nb_small, nb_big);
+      launch_getf2<T>(std::min(nb, ncol), g.cnt, st, fa, dt + g.off, nb_small, nb_big);
     else if (g.kind == L_DEEP)
-      k_deep<T, 256><<<g.cnt, 256, smem_deep(es, nb), st>>>(fa, dt + g.off, nb_small, nb_big);
+      launch_deep<T, true>(std::min(nb, ncol), g.cnt, st, fa, dt + g.off, nb_small, nb_big);
     else
       k_schur<T><<<g.cnt, TPB, smem_schur(es), st>>>(fa, dt + g.off, nb_small, nb_big);
   }
