@@ -48,8 +48,11 @@ constexpr int WV_NT = 256;
 constexpr long WV_POLL_LIMIT = 1L << 21;  // flag polls before a wait gives up
 constexpr int ST_UNIT = 2112;             // streamed tile elements (max of 32 x 65 and 64 x 33)
 constexpr int CH_UNIT = 64 * 65;          // chain tile elements
-constexpr int BWD_CH = 512;               // off-diagonal rows per backward-dot item
-constexpr int PUSH_KS = 16;               // column units (of 32) per forward-push item of a wide supernode
+// Units (32 x 64 panel tiles) that a streamed item takes one after another: a
+// level's units over ST_ITEMS items (two CTAs per SM, twice), within these
+// bounds.  Fixed items of 16 units left the upper levels with 20 to 300 items
+// of 30 to 50 us each.
+constexpr int ST_ITEMS = 4 * 148, ST_UNITS_MIN = 2, ST_UNITS_MAX = 16;
 // The right-hand sides of a pass are solved as CH_GROUPS independent chains
 // of at most CH_NR columns (more CTAs, shorter per-block products).
 constexpr int CH_NR = 4;
@@ -136,7 +139,7 @@ __device__ __forceinline__ void store_partials(T* red, const T (&acc)[NR], int x
 // = L[ncol + r, :] z_s, one 64-row block after another (narrow supernodes
 // take several blocks per item so an item streams a few units at least).
 // Backward dots (s, i, r0, slot): for the columns of block i, sum over
-// off-diagonal rows [ncol + r0, ncol + r0 + BWD_CH) of L[r, p] x_anc[r];
+// the off-diagonal rows from ncol + r0 on (32 per unit) of L[r, p] x_anc[r];
 // slot < 0 (the only chunk) writes Wb, else partial sums go to slot `slot`
 // (64 x ld each), which the backward chain item of block i adds up in chunk
 // order.
@@ -167,16 +170,18 @@ __device__ __forceinline__ StItem<T, FWD> st_item(const SolveArgs& a, int4 tk) {
     it.c0 = 0; it.clim = ncol;
     it.V = reinterpret_cast<const T*>(a.Ze) + a.c0 + (long long)first * a.ld;
     it.vlim = ncol;
-    // z = nrb | first column unit << 8; wide supernodes' items take
-    // PUSH_KS column units each (partial sums to slot w)
-    it.cb0 = tk.z >> 8;
-    it.cu = min(PUSH_KS, (ncol + 31) / 32 - it.cb0);
-    if (tk.w < 0) it.cu = (ncol + 31) / 32;
-    const int nrb = min(tk.z & 255, (nrow - it.r0 + 63) / 64);
-    it.nunits = nrb * it.cu;
+    if (tk.w < 0) {  // z = row blocks
+      it.cb0 = 0;
+      it.cu = (ncol + 31) / 32;
+      it.nunits = min(tk.z, (nrow - it.r0 + 63) / 64) * it.cu;
+    } else {  // z = 1 | column units << 3 | first column unit << 8 (partial sums to slot w)
+      it.cb0 = tk.z >> 8;
+      it.cu = min((tk.z >> 3) & 31, (ncol + 31) / 32 - it.cb0);
+      it.nunits = it.cu;
+    }
   } else {
-    it.r0 = ncol + tk.z; it.rlim = min(nrow, it.r0 + BWD_CH);
-    it.c0 = tk.y * TB; it.clim = ncol;
+    it.r0 = ncol + tk.z; it.rlim = min(nrow, it.r0 + 32 * (tk.y >> 24));  // y = block | units << 24
+    it.c0 = (tk.y & 0xffffff) * TB; it.clim = ncol;
     // the ancestors' x straight from the solution vector: row r of the item
     // is g = rs[ncol + r0 + r] (no gathered copy)
     it.V = reinterpret_cast<const T*>(a.Xg) + a.c0;
@@ -207,16 +212,18 @@ __device__ __forceinline__ void st_issue(T* S, T* Vs, const StItem<T, FWD>& it, 
     } else {
       r = rr0 + (e & 31); c = cc0 + (e >> 5); dst = (e >> 5) * 33 + (e & 31);
     }
+    // forward: columns past the block are not reduced over (nothing to fill);
+    // backward: the same for rows
     const bool ok = r < it.rlim && c < it.clim;
+    if (FWD ? c >= it.clim : r >= it.rlim) continue;
     const T* g = ok ? it.L + r + (long long)c * it.ld : it.L;
     cp_async_zfill<sizeof(T)>(S + dst, g, ok);
   }
   for (int e = threadIdx.x; e < 32 * nr; e += WV_NT) {
     const int k = e / nr, c = e - k * nr, row = vr0 + k;
-    const bool ok = row < it.vlim;
-    const long long vr = FWD ? row : (ok ? it.vrows[row] : 0);
-    const T* g = ok ? it.V + vr * ld + c : it.V;
-    cp_async_zfill<sizeof(T)>(Vs + k * NR + c, g, ok);
+    if (row >= it.vlim) break;
+    const long long vr = FWD ? row : it.vrows[row];
+    cp_async_zfill<sizeof(T)>(Vs + k * NR + c, it.V + vr * ld + c, true);
   }
 }
 
@@ -286,14 +293,21 @@ __global__ void __launch_bounds__(WV_NT) k_stream(SolveArgs a, const int4* __res
     }
     const T* S = stages + (u % NST) * SE;
     const T* V = S + ST_UNIT;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int q = 8 * g + k;
+    auto term = [&](int q) {
       const T l = FWD ? S[q * 65 + x] : S[x * 33 + q];
       T v[NR];
       lds_row<T, NR>(V + q * NR, v);
 #pragma unroll
       for (int c = 0; c < NR; ++c) acc[c] = F::fma_(l, v[c], acc[c]);
+    };
+    // reduction entries of the unit: columns (forward) or rows of the block
+    const int nq = it.vlim - 32 * (FWD ? it.cb0 + u % it.cu : u);
+    if (nq >= 32) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) term(8 * g + k);
+    } else {
+      const int qe = min(8 * g + 8, nq);
+      for (int q = 8 * g; q < qe; ++q) term(q);
     }
   }
   cp_async_wait<0>();
@@ -315,6 +329,7 @@ __global__ void __launch_bounds__(WV_NT) k_push_reduce(SolveArgs a, const int4* 
     const int r = e / nr, c = e - r * nr;
     if (r0 + r >= off) continue;
     T v = part[(long long)r * ld + c];
+#pragma unroll 8
     for (int k = 1; k < nch; ++k) v = F::add(v, part[((long long)k * 64 + r) * ld + c]);
     Us[(long long)(r0 + r) * ld + c] = v;
   }
@@ -343,7 +358,8 @@ __device__ __forceinline__ void ch_issue(T* S, const T* src, long long ld, int r
   for (int m = 0; m < 4096 / WV_NT; ++m) {
     const int e = threadIdx.x + WV_NT * m;
     const int r = e & 63, c = e >> 6;
-    const bool ok = r0 + r < rlim && c0 + c < clim;
+    if (c0 + c >= clim) break;  // (the same for a warp's lanes; columns past the block are not used)
+    const bool ok = r0 + r < rlim;
     const T* g = ok ? src + (r0 + r) + (long long)(c0 + c) * ld : src;
     cp_async_zfill<sizeof(T)>(S + c * 65 + r, g, ok);
   }
@@ -351,18 +367,23 @@ __device__ __forceinline__ void ch_issue(T* S, const T* src, long long ld, int r
 
 // acc[c] += sum over the thread's 16 reduction entries of the 64 x 64 tile
 // S (forward: S[q * 65 + x] = A[x, q]; backward: S[x * 65 + q] = A[q, x])
-// times V[q * nr + c].
+// times V[q * nr + c], q < nq.
 template <typename T, bool FWD, int NR>
-__device__ __forceinline__ void ch_tile_mv(T (&acc)[NR], const T* S, const T* V, int x, int g) {
+__device__ __forceinline__ void ch_tile_mv(T (&acc)[NR], const T* S, const T* V, int x, int g, int nq) {
   using F = Field<T>;
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const int q = 16 * g + k;
+  auto term = [&](int q) {
     const T l = FWD ? S[q * 65 + x] : S[x * 65 + q];
     T v[NR];
     lds_row<T, NR>(V + q * NR, v);
 #pragma unroll
     for (int c = 0; c < NR; ++c) acc[c] = F::fma_(l, v[c], acc[c]);
+  };
+  if (nq >= TB) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) term(16 * g + k);
+  } else {  // a narrow block (most leaves have one to a few columns)
+    const int qe = min(16 * g + 16, nq);
+    for (int q = 16 * g; q < qe; ++q) term(q);
   }
 }
 
@@ -432,12 +453,13 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
         const T* Uc = reinterpret_cast<const T*>(a.U) + a.c0 + cg0 + c;
         v = reinterpret_cast<const T*>(a.Yg)[a.c0 + cg0 + (long long)gg * ld + c];
         const int t0 = a.pull_ptr[gg], t1 = a.pull_ptr[gg + 1];
-#pragma unroll 4
+#pragma unroll 8
         for (int t = t0; t < t1; ++t) v = F::sub(v, Uc[(long long)a.pull_src[t] * ld]);
       } else {
         v = ld_cg(Ze + (long long)(i * TB + r) * ld + c);
         if (dred.y > 1) {
           T w = Wpart[(long long)r * ld + c];
+#pragma unroll 8
           for (int q = 1; q < dred.y; ++q) w = F::add(w, Wpart[((long long)q * 64 + r) * ld + c]);
           v = F::sub(v, w);
         } else if (Wb) {
@@ -462,7 +484,7 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
       Vs[e] = (c < nr && j * TB + r < ncol) ? ld_cg(Ze + (long long)(j * TB + r) * ld + c) : F::zero();
     }
     __syncthreads();
-    ch_tile_mv<T, FWD, NR>(acc, S, Vs, x, g);
+    ch_tile_mv<T, FWD, NR>(acc, S, Vs, x, g, min(TB, ncol - j * TB));
     __syncthreads();  // tile and right-hand sides consumed
     if (u + 1 < nd) issue(u + 1);
     cp_async_commit();
@@ -478,7 +500,7 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
     wv[e] = (r < nb && c < nr) ? F::sub(wv[e], slice_sum<T, NR>(red, r, c)) : F::zero();
   }
   __syncthreads();
-  ch_tile_mv<T, FWD, NR>(acc, Lv, wv, x, g);
+  ch_tile_mv<T, FWD, NR>(acc, Lv, wv, x, g, nb);
   store_partials<T, NR>(red, acc, x, g);
   __syncthreads();
   for (int e = tid; e < 64 * nr; e += WV_NT) {

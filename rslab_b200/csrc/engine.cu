@@ -872,23 +872,35 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
         W.ntasks = (int)(H.st4.size() - W.task_off);
         H.fwdplan.push_back(W);
       }
-      // push items: 64-row blocks, several per item for narrow supernodes
-      // (about 8 column units per item)
-      // (wide supernodes: PUSH_KS column units per item, partial sums
-      // reduced in chunk order by the next launch)
+      // push items: 64-row blocks of a supernode, several per item for narrow
+      // supernodes, and column chunks for wide ones (partial sums reduced in
+      // chunk order by the next launch).  An item streams its units one after
+      // another, so a level's units are cut into about ST_ITEMS items of
+      // ST_UNITS_MIN to ST_UNITS_MAX units
+      long long units_f = 0, units_b = 0;
+      for (int64_t s : lvl) {
+        const long long nc = S.sn[s].ncol, off = H.nrow[s] - nc;
+        units_f += (off + 63) / 64 * ((nc + 31) / 32);
+        units_b += (off + 31) / 32 * ((nc + TB - 1) / TB);
+      }
+      auto units_per_item = [](long long units) {
+        return (int)std::min<long long>(ST_UNITS_MAX, std::max<long long>(ST_UNITS_MIN, units / ST_ITEMS));
+      };
       Launch Pu{L_FWD_PUSH, (long long)H.st4.size(), 0, 0};
       std::vector<int4> pred;
       int pslot = 0;
+      const int ks = units_per_item(units_f), bch = 32 * units_per_item(units_b);
       for (int64_t s : lvl) {
         const int cu = (int)((S.sn[s].ncol + 31) / 32), off = H.nrow[s] - (int)S.sn[s].ncol;
-        if (cu <= PUSH_KS) {
-          const int nrb = std::max(1, 8 / cu);
+        if (cu <= ks) {
+          const int nrb = std::max(1, std::min(8, ks) / cu);
           for (int r0 = 0; r0 < off; r0 += 64 * nrb) H.st4.push_back(make_int4((int)s, r0, nrb, -1));
         } else {
-          const int nch = (cu + PUSH_KS - 1) / PUSH_KS;
+          const int nch = (cu + ks - 1) / ks;
           for (int r0 = 0; r0 < off; r0 += 64) {
             pred.push_back(make_int4((int)s, r0, pslot, nch));
-            for (int q = 0; q < nch; ++q) H.st4.push_back(make_int4((int)s, r0, 1 | ((q * PUSH_KS) << 8), pslot + q));
+            for (int q = 0; q < nch; ++q)
+              H.st4.push_back(make_int4((int)s, r0, 1 | (ks << 3) | ((q * ks) << 8), pslot + q));
             pslot += nch;
           }
         }
@@ -910,13 +922,14 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
       for (int64_t s : lvl) {
         const int off = H.nrow[s] - (int)S.sn[s].ncol;
         if (off <= 0) continue;
-        const int nch = (off + BWD_CH - 1) / BWD_CH;
+        const int nch = (off + bch - 1) / bch;
         if (nch > 1) H.dots_red[s] = make_int2(slot, nch);
         for (int i = 0; i * TB < S.sn[s].ncol; ++i) {
+          const int w = i | (bch / 32) << 24;
           if (nch == 1) {
-            H.st4.push_back(make_int4((int)s, i, 0, -1));
+            H.st4.push_back(make_int4((int)s, w, 0, -1));
           } else {
-            for (int q = 0; q < nch; ++q) H.st4.push_back(make_int4((int)s, i, q * BWD_CH, slot + q));
+            for (int q = 0; q < nch; ++q) H.st4.push_back(make_int4((int)s, w, q * bch, slot + q));
             slot += nch;
           }
         }
@@ -1123,8 +1136,10 @@ struct rslab_fac_handle {
   double factor_ms = 0, solve_ms = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // side stream of the factor (lowest priority) and its fork / join events
-  cudaStream_t st2 = nullptr, st3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_cm[2] = {nullptr, nullptr};
+  // (st2: Schur update beyond the next block, st3: early descendant updates,
+  // st4: inverse diagonal blocks, which only the solves read)
+  cudaStream_t st2 = nullptr, st3 = nullptr, st4 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_inv = nullptr, ev_cm[2] = {nullptr, nullptr};
   // per-launch rows of the last factor/solve profile
   std::vector<int> tr_kind, tr_grid;
   std::vector<float> tr_ms;
@@ -1144,6 +1159,8 @@ struct rslab_fac_handle {
       if (e) cudaEventDestroy(e);
     if (st2) cudaStreamDestroy(st2);
     if (st3) cudaStreamDestroy(st3);
+    if (st4) cudaStreamDestroy(st4);
+    if (ev_inv) cudaEventDestroy(ev_inv);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (own_stream && st) cudaStreamDestroy(st);
@@ -1278,7 +1295,7 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
       default: return true;
     }
   };
-  bool cm_pending[2] = {false, false};
+  bool cm_pending[2] = {false, false}, inv_pending = false;
   for (const Launch& L : H.fplan) {
     if (!runs(L)) continue;
     cudaStream_t ls = st;
@@ -1288,7 +1305,16 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
       cm_pending[L.nb_slot & 1] = false;
       continue;
     }
-    if (overlap && L.side == 2) {
+    if (overlap && L.kind == L_DIAG_INV) {
+      // a level's inverses overlap the levels above (in line they took 2-8% of
+      // a factor: 30 launches, 1.5 ms, at 64^3)
+      if (side_pending) CK(cudaStreamWaitEvent(st, F.ev_join, 0));
+      side_pending = false;
+      CK(cudaEventRecord(F.ev_fork, st));
+      CK(cudaStreamWaitEvent(F.st4, F.ev_fork, 0));
+      ls = F.st4;
+      inv_pending = true;
+    } else if (overlap && L.side == 2) {
       CK(cudaEventRecord(F.ev_fork, st));
       CK(cudaStreamWaitEvent(F.st3, F.ev_fork, 0));
       ls = F.st3;
@@ -1392,12 +1418,16 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
     if (ls == F.st3) {
       CK(cudaEventRecord(F.ev_cm[L.nb_slot & 1], ls));
       cm_pending[L.nb_slot & 1] = true;
-    } else if (ls != st) {
+    } else if (ls == F.st2) {
       CK(cudaEventRecord(F.ev_join, ls));
       side_pending = true;
     }
   }
   if (side_pending) CK(cudaStreamWaitEvent(st, F.ev_join, 0));
+  if (inv_pending) {
+    CK(cudaEventRecord(F.ev_inv, F.st4));
+    CK(cudaStreamWaitEvent(st, F.ev_inv, 0));
+  }
   for (int q = 0; q < 2; ++q)
     if (cm_pending[q]) CK(cudaStreamWaitEvent(st, F.ev_cm[q], 0));
   if (F.set.drop_tol > 0.0 && H.ns > 0) k_drop_tol<T><<<H.ns, 256, 0, st>>>(fa, F.set.drop_tol);
@@ -2283,6 +2313,8 @@ static int factor_impl(rslab_sym_handle* sym, int dtype, int dtype_hi, const voi
     }
     CK(cudaStreamCreateWithPriority(&F->st2, cudaStreamNonBlocking, prio_lo));
     CK(cudaStreamCreateWithPriority(&F->st3, cudaStreamNonBlocking, prio_lo));
+    CK(cudaStreamCreateWithPriority(&F->st4, cudaStreamNonBlocking, prio_lo));
+    CK(cudaEventCreateWithFlags(&F->ev_inv, cudaEventDisableTiming));
     for (cudaEvent_t& e : F->ev_cm) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaEventCreate(&F->ev0));
     CK(cudaEventCreate(&F->ev1));
