@@ -43,8 +43,8 @@ struct SolveArgs {
   const void* dsub;
   const unsigned char* kind;
   const int* lperm;
-  void* Yg;   // n x ld, g order
-  void* Ze;   // n x ld, e order
+  void* Yg;   // n x ld: forward the right-hand sides (g order), backward D^-1 z (e order)
+  void* Ze;   // n x ld, e order: z, then x; all-ones bits until the value is known
   void* Xg;   // n x ld, g order
   void* U;    // sum_s (nrow_s - ncol_s) x ld: U_s = L21_s z_s
   void* Wb;   // n x ld, e order: backward off-diagonal dots
@@ -55,21 +55,38 @@ struct SolveArgs {
   const void* linv;       // inverses of the TB x TB diagonal blocks of wide supernodes
   const long long* linv_off;
   void* Wp;               // slots x 32 x ld partial sums of the split backward dots
-  int* wstate;            // wavefront solves: status, abort word, ticket counters, block flags
+  int* wstate;            // chain solves: status, abort word, ticket counters
   int ld;     // row stride (total rhs count)
   int c0;     // first rhs column of this pass
   int nrhs;   // rhs columns in this pass (<= RHS_MAX)
 };
 
-// Yg[g] = s[perm[g]] * b[perm[g]] (scaled, permuted in).
+// The initial pattern of the published vector: every bit set.
+template <typename T>
+__device__ __forceinline__ T unpublished() {
+  using R = typename Field<T>::Real;
+  R r;
+  if constexpr (sizeof(R) == 8)
+    r = __longlong_as_double(-1ll);
+  else
+    r = __int_as_float(-1);
+  if constexpr (Field<T>::complex)
+    return T{r, r};
+  else
+    return r;
+}
+
+// Yg[g] = s[perm[g]] * b[perm[g]] (scaled, permuted in), and the published
+// vector reset.
 template <typename T>
 __global__ void k_perm_in(int n, int nrhs, const int* __restrict__ perm, const double* __restrict__ s,
-                          const T* __restrict__ b, T* __restrict__ Yg) {
+                          const T* __restrict__ b, T* __restrict__ Yg, T* __restrict__ Ze) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= (long long)n * nrhs) return;
   int g = (int)(idx / nrhs), c = (int)(idx % nrhs);
   int i = perm[g];
   Yg[idx] = Field<T>::scale(b[(long long)i * nrhs + c], s[i]);
+  Ze[idx] = unpublished<T>();
 }
 
 // x[perm[g]] = s[perm[g]] * Xg[g] (permuted out, scaled back).
@@ -151,7 +168,9 @@ __global__ void __launch_bounds__(DI_NT) k_diag_inv(const int2* __restrict__ tas
 }
 
 // D^-1 on the e-indexed forward solution, after the whole forward sweep
-// (ancestors' gathers need z, not D^-1 z).  1x1 and 2x2 blocks.
+// (ancestors' gathers need z, not D^-1 z), into Yg (the right-hand sides are
+// used up); the published vector is reset for the backward sweep.  1x1 and
+// 2x2 blocks.
 template <typename T>
 __global__ void k_dsolve(int n, SolveArgs a) {
   using F = Field<T>;
@@ -161,19 +180,22 @@ __global__ void k_dsolve(int n, SolveArgs a) {
   const T* d = reinterpret_cast<const T*>(a.d);
   const T* ds = reinterpret_cast<const T*>(a.dsub);
   T* Z = reinterpret_cast<T*>(a.Ze) + a.c0;
+  T* W = reinterpret_cast<T*>(a.Yg) + a.c0;
   const unsigned char kd = a.kind[e];
   if (kd == 0) {
-    T* z = Z + (long long)e * a.ld + c;
-    *z = F::mul(*z, F::recip(d[e]));
+    const long long o = (long long)e * a.ld + c;
+    W[o] = F::mul(Z[o], F::recip(d[e]));
+    Z[o] = unpublished<T>();
   } else if (kd == 1) {
     T d11 = d[e], d21 = ds[e], d22 = d[e + 1];
     T det = F::sub(F::mul(d11, d22), F::mul(d21, d21));
     T di = F::recip(det);
-    T* z0 = Z + (long long)e * a.ld + c;
-    T* z1 = Z + (long long)(e + 1) * a.ld + c;
-    T a0 = *z0, a1 = *z1;
-    *z0 = F::mul(F::sub(F::mul(d22, a0), F::mul(d21, a1)), di);
-    *z1 = F::mul(F::sub(F::mul(d11, a1), F::mul(d21, a0)), di);
+    const long long o0 = (long long)e * a.ld + c, o1 = o0 + a.ld;
+    const T a0 = Z[o0], a1 = Z[o1];
+    W[o0] = F::mul(F::sub(F::mul(d22, a0), F::mul(d21, a1)), di);
+    W[o1] = F::mul(F::sub(F::mul(d11, a1), F::mul(d21, a0)), di);
+    Z[o0] = unpublished<T>();
+    Z[o1] = unpublished<T>();
   }
 }
 

@@ -26,15 +26,18 @@
 //   backward: x_i = Linv_i^T (w_i - W_i - sum_{j>i, descending} L_ji^T x_j)
 // with Linv_i the precomputed inverse of the unit-lower diagonal block and
 // W_i the off-diagonal dots.  The 64 x 64 tiles stream through shared
-// memory ahead of the chain; z_j / x_j are read (L2 only) after block j's
-// flag.  Items are handed out in ticket order (an atomic counter per launch,
-// not blockIdx) and every item waits only on items with smaller tickets,
-// whose CTAs have therefore started, so the chain progresses whatever the
-// number of resident CTAs.  A finished block is published by one thread
-// after a CTA barrier: fence, then a gpu-scope release store of the flag; a
-// waiting CTA polls with acquire loads a bounded number of times and on
-// timeout raises the launch-wide abort word and a sticky status that the
-// host reads after the solve.
+// memory ahead of the chain.  Items are handed out in ticket order (an
+// atomic counter per launch, not blockIdx) and every item waits only on items
+// with smaller tickets, whose CTAs have therefore started, so the chain
+// progresses whatever the number of resident CTAs.  A block's values are
+// their own flags: the vector starts out as a bit pattern that no result has
+// (all ones; a NaN result is stored as the quiet NaN), every value is stored
+// with a gpu-scope relaxed store, and a waiting thread polls the values it
+// needs (relaxed loads of the same width).  One round trip through L2 per
+// block, against three (release fence, flag, value) with a flag per block:
+// 64^3 root, 64 blocks, 231 us with flags.  Polls are bounded; on a
+// timeout the thread raises the launch-wide abort word and a sticky status
+// that the host reads after the solve.
 // Reference: the column-block substitution of solve_ldlt_block
 // (src/dense/ldlt_generic.rs:618-714), reorganised as a dependency chain.
 #pragma once
@@ -45,7 +48,7 @@
 namespace rsd {
 
 constexpr int WV_NT = 256;
-constexpr long WV_POLL_LIMIT = 1L << 21;  // flag polls before a wait gives up
+constexpr long WV_POLL_LIMIT = 1L << 21;  // polls before a wait gives up
 constexpr int ST_UNIT = 2112;             // streamed tile elements (max of 32 x 65 and 64 x 33)
 constexpr int CH_UNIT = 64 * 65;          // chain tile elements
 // Units (32 x 64 panel tiles) that a streamed item takes one after another: a
@@ -91,32 +94,65 @@ __host__ __device__ constexpr size_t ch_smem_bytes(int nr) {
 
 // Wave state (ints): [0] sticky status (nonzero after a timed-out wait;
 // cleared by the host when read), then the per-pass region cleared before
-// every pass: [1] abort word, [2, 2 + nchain) ticket counters, then the
-// forward and the backward block flags.
+// every pass: [1] abort word, [2, 2 + nchain) ticket counters.
 constexpr int WV_STATE_ABORT = 1;
 constexpr int WV_STATE_CTR = 2;
 
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// Published values: relaxed gpu-scope stores and loads of one word per
+// component group (c32 as one 8-byte word, c64 as two); false from
+// ld_published while the value is still the initial pattern.
+__device__ __forceinline__ void st_word(unsigned* p, unsigned v) {
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_word(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned ld_word(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned quiet_bits(float v) { return v != v ? 0x7fc00000u : __float_as_uint(v); }
+__device__ __forceinline__ unsigned long long quiet_bits(double v) {
+  return v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v);
+}
+__device__ __forceinline__ void st_published(float* p, float v) { st_word(reinterpret_cast<unsigned*>(p), quiet_bits(v)); }
+__device__ __forceinline__ void st_published(double* p, double v) {
+  st_word(reinterpret_cast<unsigned long long*>(p), quiet_bits(v));
+}
+__device__ __forceinline__ void st_published(c32* p, c32 v) {
+  st_word(reinterpret_cast<unsigned long long*>(p),
+          (unsigned long long)quiet_bits(v.im) << 32 | quiet_bits(v.re));
+}
+__device__ __forceinline__ void st_published(c64* p, c64 v) {
+  st_published(&p->re, v.re);
+  st_published(&p->im, v.im);
+}
+__device__ __forceinline__ bool ld_published(const float* p, float& v) {
+  const unsigned w = ld_word(reinterpret_cast<const unsigned*>(p));
+  v = __uint_as_float(w);
+  return w != ~0u;
+}
+__device__ __forceinline__ bool ld_published(const double* p, double& v) {
+  const unsigned long long w = ld_word(reinterpret_cast<const unsigned long long*>(p));
+  v = __longlong_as_double((long long)w);
+  return w != ~0ull;
+}
+__device__ __forceinline__ bool ld_published(const c32* p, c32& v) {
+  const unsigned long long w = ld_word(reinterpret_cast<const unsigned long long*>(p));
+  v = c32{__uint_as_float((unsigned)w), __uint_as_float((unsigned)(w >> 32))};
+  return w != ~0ull;
+}
+__device__ __forceinline__ bool ld_published(const c64* p, c64& v) {
+  const bool a = ld_published(&p->re, v.re), b = ld_published(&p->im, v.im);
+  return a && b;
 }
 __device__ __forceinline__ int ld_volatile(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
-
-// L2-only loads of vectors written by other CTAs of the same launch.
-__device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
-__device__ __forceinline__ float ld_cg(const float* p) { return __ldcg(p); }
-__device__ __forceinline__ c64 ld_cg(const c64* p) {
-  const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
-  return c64{v.x, v.y};
-}
-__device__ __forceinline__ c32 ld_cg(const c32* p) {
-  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-  return c32{v.x, v.y};
-}
 
 // Slice partials live at red[(g * NR + c) * 65 + x] (lanes over x write
 // consecutive words).  The sum over g = 0..3 in order:
@@ -336,14 +372,15 @@ __global__ void __launch_bounds__(WV_NT) k_push_reduce(SolveArgs a, const int4* 
 }
 
 // ---------------------------------------------------------------------------
-// Chain items (s, 0 / 1 = forward / backward, block i, first flag of s).
+// Chain items (s, direction | 2 column group, block i, -); direction 0 = forward, 1 = backward.
 // ---------------------------------------------------------------------------
 
-// Wait (thread 0) until flag `f` is set; false on timeout or abort.
-__device__ __forceinline__ bool wv_wait(const int* flags, int f, int* state) {
+// Wait until *p is published; false on timeout or abort.
+template <typename T>
+__device__ __forceinline__ bool wv_wait(const T* p, T& v, int* state) {
   for (long it = 0; it < WV_POLL_LIMIT; ++it) {
-    if (ld_acquire_gpu(flags + f) != 0) return true;
-    if (ld_volatile(state + WV_STATE_ABORT) != 0) return false;
+    if (ld_published(p, v)) return true;
+    if ((it & 15) == 15 && ld_volatile(state + WV_STATE_ABORT) != 0) return false;
   }
   atomicExch(state + WV_STATE_ABORT, 1);
   atomicExch(state, 1);
@@ -391,11 +428,10 @@ __device__ __forceinline__ void ch_tile_mv(T (&acc)[NR], const T* S, const T* V,
 // pass for the levels whose items already fill the GPU: one CTA per block
 // then reads the block's inverse and dependency tiles once).
 template <typename T, bool FWD, int NR>
-__global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __restrict__ tasks, int ctr, int flag_base,
-                                                 int gw) {
+__global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __restrict__ tasks, int ctr, int gw) {
   using F = Field<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int sh_t, sh_abort;
+  __shared__ int sh_t;
   const int ld = a.ld;
   T* S = reinterpret_cast<T*>(smem_raw);  // dependency tile; later the slice partials (4 x NR x 65)
   T* red = S;
@@ -403,22 +439,17 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
   T* Vs = Lv + CH_UNIT;                   // 64 x NR
   T* wv = Vs + 64 * NR;                   // 64 x NR
   const int tid = threadIdx.x, x = tid & 63, g = tid >> 6;
-  if (tid == 0) {
-    sh_t = atomicAdd(a.wstate + WV_STATE_CTR + ctr, 1);
-    sh_abort = 0;
-  }
+  if (tid == 0) sh_t = atomicAdd(a.wstate + WV_STATE_CTR + ctr, 1);
   __syncthreads();
   if (ld_volatile(a.wstate + WV_STATE_ABORT) != 0) return;
   const int4 tk = tasks[sh_t];
-  const int s = tk.x, i = tk.z, fb = tk.w;
+  const int s = tk.x, i = tk.z;
   // column group: columns [cg0, cg0 + nr) of the pass; a group with no
   // columns in this pass has nothing to do (its dependents are in the same
   // group)
   const int cg0 = gw * (tk.y >> 1);
   const int nr = min(gw, a.nrhs - cg0);
   if (nr <= 0) return;
-  // flags of group g: flag index (fb + block) * CH_GROUPS + g
-  int* flags = a.wstate + flag_base + (long long)fb * CH_GROUPS + (tk.y >> 1);
   const int first = a.sn_first[s], ncol = a.sn_ncol[s], nrow = a.sn_nrow[s];
   const int nblk = (ncol + TB - 1) / TB, nb = min(TB, ncol - i * TB);
   const T* L = reinterpret_cast<const T*>(a.panel) + a.sn_poff[s];
@@ -431,6 +462,17 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
     const int j = dep(u);
     if (FWD) ch_issue<T>(S, L, nrow, i * TB, ncol, j * TB, ncol);
     else ch_issue<T>(S, L, nrow, j * TB, ncol, i * TB, ncol);
+    // the tile after it into L2 (one tile fits in shared memory)
+    if (u + 1 < nd) {
+      const int jn = dep(u + 1);
+      const int pr = FWD ? i * TB : jn * TB, pc = FWD ? jn * TB : i * TB;
+      constexpr int LPC = TB * (int)sizeof(T) / 128;  // cache lines of a tile column
+      for (int e = tid; e < TB * LPC; e += WV_NT) {
+        const int c = pc + e / LPC, r = pr + (e % LPC) * (128 / (int)sizeof(T));
+        if (c < ncol && r < ncol)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(L + r + (long long)c * nrow));
+      }
+    }
   };
   ch_issue<T>(Lv, Li, ncol <= TB ? ncol : TB, 0, nb, 0, nb);
   if (nd > 0) issue(0);
@@ -442,6 +484,7 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
   // (W_i = off-diagonal dots; for a supernode whose dots were split into
   // row chunks, the chunk partials summed here in chunk order).
   const T* Wb = (!FWD && nrow > ncol) ? reinterpret_cast<const T*>(a.Wb) + a.c0 + cg0 + (long long)first * ld : nullptr;
+  const T* Wd = reinterpret_cast<const T*>(a.Yg) + a.c0 + cg0 + (long long)first * ld;  // backward: D^-1 z
   const int2 dred = FWD ? make_int2(0, 0) : a.dots_red[s];
   const T* Wpart = reinterpret_cast<const T*>(a.Wp) + (long long)(dred.x + i * dred.y) * 64 * ld + cg0;
   for (int e = tid; e < 64 * NR; e += WV_NT) {
@@ -456,7 +499,7 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
 #pragma unroll 8
         for (int t = t0; t < t1; ++t) v = F::sub(v, Uc[(long long)a.pull_src[t] * ld]);
       } else {
-        v = ld_cg(Ze + (long long)(i * TB + r) * ld + c);
+        v = Wd[(long long)(i * TB + r) * ld + c];
         if (dred.y > 1) {
           T w = Wpart[(long long)r * ld + c];
 #pragma unroll 8
@@ -475,15 +518,22 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
 #pragma unroll 1
   for (int u = 0; u < nd; ++u) {
     const int j = dep(u);
-    if (tid == 0 && !wv_wait(flags, j * CH_GROUPS, a.wstate)) sh_abort = 1;
-    cp_async_wait<0>();
-    __syncthreads();  // tile u landed; flag j observed
-    if (sh_abort) return;
+    bool bad = false;
+    if (nd - u > 2) {
+      // not next in line: one thread waits, so that the blocks far behind
+      // leave the values' cache lines to the ones about to use them
+      T v;
+      if (tid == 0) bad = !wv_wait(Ze + (long long)(min((j + 1) * TB, ncol) - 1) * ld, v, a.wstate);
+      if (__syncthreads_or(bad)) return;
+    }
     for (int e = tid; e < 64 * NR; e += WV_NT) {
       const int r = e / NR, c = e % NR;
-      Vs[e] = (c < nr && j * TB + r < ncol) ? ld_cg(Ze + (long long)(j * TB + r) * ld + c) : F::zero();
+      T v = F::zero();
+      if (!bad && c < nr && j * TB + r < ncol) bad = !wv_wait(Ze + (long long)(j * TB + r) * ld + c, v, a.wstate);
+      Vs[e] = v;
     }
-    __syncthreads();
+    cp_async_wait<0>();
+    if (__syncthreads_or(bad)) return;  // tile u and block j are here
     ch_tile_mv<T, FWD, NR>(acc, S, Vs, x, g, min(TB, ncol - j * TB));
     __syncthreads();  // tile and right-hand sides consumed
     if (u + 1 < nd) issue(u + 1);
@@ -507,16 +557,12 @@ __global__ void __launch_bounds__(WV_NT) k_chain(SolveArgs a, const int4* __rest
     const int r = e / nr, c = e - r * nr;
     if (r >= nb) continue;
     const T v = slice_sum<T, NR>(red, r, c);
-    Ze[(long long)(i * TB + r) * ld + c] = v;
+    st_published(Ze + (long long)(i * TB + r) * ld + c, v);
     if (!FWD) {
       T* Xw = reinterpret_cast<T*>(a.Xg) + a.c0 + cg0;
       Xw[(long long)(first + a.lperm[first + i * TB + r]) * ld + c] = v;
     }
   }
-  __syncthreads();
-  // the release store orders the CTA's stores above (barrier, then a
-  // cumulative gpu-scope release)
-  if (tid == 0) st_release_gpu(flags + (long long)i * CH_GROUPS, 1);
 }
 
 }  // namespace rsd

@@ -191,10 +191,7 @@ struct rslab_sym_handle {
   int bwd_slots = 0;                  // partial-sum slots of the split push / backward dots (max per level)
   std::vector<long long> linv_off;    // wide supernodes: inverses of their TB x TB diagonal blocks
   long long linv_elems = 0;
-  // chain solves: per wide supernode the index of its block-0 flag (-1 for
-  // narrow ones), flags per direction, and ticket counters (launches)
-  std::vector<int> flag_off;
-  int nflags = 0, nwave = 0;
+  int nwave = 0;  // chain solves: ticket counters (launches)
   std::vector<int> t1;
   std::vector<int2> t2;
   std::vector<int4> st4;  // blocked diagonal-solve tasks (s, j0, r0 | c0, 0)
@@ -566,13 +563,7 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
     H.linv_off[s] = H.linv_elems;
     H.linv_elems += linv_elems_of((int)S.sn[s].ncol);
   }
-  H.flag_off.assign(ns, -1);
-  H.nflags = 0;
   H.nwave = 0;
-  for (int s = 0; s < ns; ++s) {
-    H.flag_off[s] = H.nflags;
-    H.nflags += (int)((S.sn[s].ncol + TB - 1) / TB);
-  }
   // Pull lists: every off-diagonal row r of updater k (U row uoff[k] + r)
   // lands on one column g of an ancestor; list the pushes per g in the
   // ancestor's update-list order so the gather subtracts them in that order.
@@ -868,7 +859,7 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
         for (int b = 0; b < maxb; ++b)
           for (int64_t s : lvl)
             if (b * TB < S.sn[s].ncol)
-              for (int g = 0; g < ngroups; ++g) H.st4.push_back(make_int4((int)s, 2 * g, b, H.flag_off[s]));
+              for (int g = 0; g < ngroups; ++g) H.st4.push_back(make_int4((int)s, 2 * g, b, 0));
         W.ntasks = (int)(H.st4.size() - W.task_off);
         H.fwdplan.push_back(W);
       }
@@ -945,7 +936,7 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
             const int nblk = (int)((S.sn[s].ncol + TB - 1) / TB);
             if (dd < nblk)
               for (int g = 0; g < ngroups; ++g)
-                H.st4.push_back(make_int4((int)s, 1 + 2 * g, nblk - 1 - dd, H.flag_off[s]));
+                H.st4.push_back(make_int4((int)s, 1 + 2 * g, nblk - 1 - dd, 0));
           }
         W.ntasks = (int)(H.st4.size() - W.task_off);
         bw.push_back(W);
@@ -1016,31 +1007,31 @@ void solve_nr_attrs() {
 // Launch a streamed (kind 0) or chain (kind 1) solve kernel instantiated for
 // the smallest NR in {1, 4, RHS_MAX} that holds nr columns.
 template <typename T, bool FWD, int NR>
-void launch_solve_nr(int kind, int grid, int nr, const SolveArgs& sa, const int4* tasks, int ctr, int flags,
+void launch_solve_nr(int kind, int grid, int nr, const SolveArgs& sa, const int4* tasks, int ctr,
                      cudaStream_t st, int gw = CH_NR) {
   if (kind == 0)
     k_stream<T, FWD, NR><<<grid, WV_NT, st_smem_bytes<T>(NR), st>>>(sa, tasks);
   else
-    k_chain<T, FWD, NR><<<grid, WV_NT, ch_smem_bytes<T>(NR), st>>>(sa, tasks, ctr, flags, gw);
+    k_chain<T, FWD, NR><<<grid, WV_NT, ch_smem_bytes<T>(NR), st>>>(sa, tasks, ctr, gw);
 }
 template <typename T, bool FWD>
-void launch_solve(int kind, int grid, int nr, const SolveArgs& sa, const int4* tasks, int ctr = 0, int flags = 0,
+void launch_solve(int kind, int grid, int nr, const SolveArgs& sa, const int4* tasks, int ctr = 0,
                   cudaStream_t st = nullptr, bool wide = false) {
   if (kind == 1) {  // chain items carry at most CH_NR columns each, or all of them (wide levels)
     if (nr <= 1)
-      launch_solve_nr<T, FWD, 1>(kind, grid, nr, sa, tasks, ctr, flags, st);
+      launch_solve_nr<T, FWD, 1>(kind, grid, nr, sa, tasks, ctr, st);
     else if (nr <= CH_NR || !wide)
-      launch_solve_nr<T, FWD, CH_NR>(kind, grid, nr, sa, tasks, ctr, flags, st);
+      launch_solve_nr<T, FWD, CH_NR>(kind, grid, nr, sa, tasks, ctr, st);
     else
-      launch_solve_nr<T, FWD, RHS_MAX>(kind, grid, nr, sa, tasks, ctr, flags, st, RHS_MAX);
+      launch_solve_nr<T, FWD, RHS_MAX>(kind, grid, nr, sa, tasks, ctr, st, RHS_MAX);
     return;
   }
   if (nr <= 1)
-    launch_solve_nr<T, FWD, 1>(kind, grid, nr, sa, tasks, ctr, flags, st);
+    launch_solve_nr<T, FWD, 1>(kind, grid, nr, sa, tasks, ctr, st);
   else if (nr <= 4)
-    launch_solve_nr<T, FWD, 4>(kind, grid, nr, sa, tasks, ctr, flags, st);
+    launch_solve_nr<T, FWD, 4>(kind, grid, nr, sa, tasks, ctr, st);
   else
-    launch_solve_nr<T, FWD, RHS_MAX>(kind, grid, nr, sa, tasks, ctr, flags, st);
+    launch_solve_nr<T, FWD, RHS_MAX>(kind, grid, nr, sa, tasks, ctr, st);
 }
 
 template <typename T>
@@ -1125,7 +1116,7 @@ struct rslab_fac_handle {
   int ws_nrhs = 0;
   void *Yg = nullptr, *Ze = nullptr, *Xg = nullptr, *Ub = nullptr, *Wb = nullptr, *bdev = nullptr, *xdev = nullptr;
   void* Wp = nullptr;  // partial sums of the split backward dots
-  int* wstate = nullptr;   // wavefront solves: sticky status, abort word, ticket counters, block flags
+  int* wstate = nullptr;   // chain solves: sticky status, abort word, ticket counters
   int* h_wstat = nullptr;  // pinned copy of the sticky status after each solve
   std::vector<std::unique_ptr<void, DFree>> ws;
   cudaGraphExec_t sgraph = nullptr;
@@ -1487,9 +1478,9 @@ void run_factor(rslab_fac_handle& F) {
 }
 
 // Wave state: sticky status, abort word, one ticket counter per wavefront
-// launch, forward and backward block flags.
+// launch.
 size_t wave_state_ints(const rslab_sym_handle& H) {
-  return (size_t)WV_STATE_CTR + H.nwave + 2 * (size_t)CH_GROUPS * H.nflags;
+  return (size_t)WV_STATE_CTR + H.nwave;
 }
 
 // After a synchronised solve: a timed-out wavefront wait (sticky status set
@@ -1581,23 +1572,22 @@ void enqueue_solve(rslab_fac_handle& F, const T* b, T* x, int nrhs, Prof* prof =
   const int n = H.n;
   cudaStream_t st = F.st;
   if (prof) prof->mark(st, -1);
-  k_perm_in<T><<<grid1((long long)n * nrhs), 256, 0, st>>>(n, nrhs, H.d_perm, F.scale, b, (T*)F.Yg);
+  k_perm_in<T><<<grid1((long long)n * nrhs), 256, 0, st>>>(n, nrhs, H.d_perm, F.scale, b, (T*)F.Yg, (T*)F.Ze);
   if (prof) prof->mark(st, 0);
   for (int c0 = 0; c0 < nrhs; c0 += RHS_MAX) {
     const int nr = std::min(RHS_MAX, nrhs - c0);
     SolveArgs sa = make_sargs<T>(F, nrhs, c0, nr);
     CK(cudaMemsetAsync(F.wstate + 1, 0, (wave_state_ints(H) - 1) * sizeof(int), st));
-    const int fwd_flags = WV_STATE_CTR + H.nwave, bwd_flags = fwd_flags + CH_GROUPS * H.nflags;
     for (const Launch& L : H.fwdplan) {
       switch (L.kind) {
         case L_FWD_CHAIN:
-          launch_solve<T, true>(1, L.ntasks, nr, sa, H.d_st4 + L.task_off, L.nb_slot, fwd_flags, st, L.narrow != 0);
+          launch_solve<T, true>(1, L.ntasks, nr, sa, H.d_st4 + L.task_off, L.nb_slot, st, L.narrow != 0);
           break;
         case L_FWD_PUSH_RED:
           k_push_reduce<T><<<L.ntasks, WV_NT, 0, st>>>(sa, H.d_st4 + L.task_off);
           break;
         default:
-          launch_solve<T, true>(0, L.ntasks, nr, sa, H.d_st4 + L.task_off, 0, 0, st);
+          launch_solve<T, true>(0, L.ntasks, nr, sa, H.d_st4 + L.task_off, 0, st);
       }
       if (prof) prof->mark(st, (L.kind == L_FWD_PUSH || L.kind == L_FWD_PUSH_RED) ? 2 : 1, L.ntasks, L.kind);
     }
@@ -1606,10 +1596,10 @@ void enqueue_solve(rslab_fac_handle& F, const T* b, T* x, int nrhs, Prof* prof =
     for (const Launch& L : H.bwdplan) {
       switch (L.kind) {
         case L_BWD_OFF:
-          launch_solve<T, false>(0, L.ntasks, nr, sa, H.d_st4 + L.task_off, 0, 0, st);
+          launch_solve<T, false>(0, L.ntasks, nr, sa, H.d_st4 + L.task_off, 0, st);
           break;
         default:  // L_BWD_CHAIN
-          launch_solve<T, false>(1, L.ntasks, nr, sa, H.d_st4 + L.task_off, L.nb_slot, bwd_flags, st, L.narrow != 0);
+          launch_solve<T, false>(1, L.ntasks, nr, sa, H.d_st4 + L.task_off, L.nb_slot, st, L.narrow != 0);
       }
       if (prof)
         prof->mark(st, (L.kind == L_BWD_OFF || L.kind == L_BWD_OFF_RED || L.kind == L_BWD_GATHER) ? 4 : 5, L.ntasks,
