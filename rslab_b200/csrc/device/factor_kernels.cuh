@@ -25,9 +25,11 @@ namespace rsd {
 
 constexpr int TILE = 64;      // output tile edge of the GEMM-class kernels
 constexpr int TPB = 256;      // threads per CTA of the GEMM-class kernels
-// Deep rows that getf2 solves itself: two passes of its eight warps (10 us)
-// against a launch of k_deep (about 8 us with the launch); 192 rows took six.
-constexpr int FUSE_DEEP_ROWS = 64;
+// Deep rows that getf2 solves itself, for blocks of at most FUSE_PW columns:
+// two passes of its eight warps (10 us) against a launch of k_deep (about 8 us
+// with the launch); 192 rows took six.  A pass over 128 columns takes 45 us
+// (c32), so wider blocks always leave them to k_deep.
+constexpr int FUSE_DEEP_ROWS = 64, FUSE_PW = 64;
 constexpr int EA_ROWS = 1024;        // front rows per extend-add task
 struct FactorArgs {
   // structure (device)

@@ -391,7 +391,15 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       } else {
         double v = -1.0;
         int idx = INT_MAX;
-        for (int i = c + 1 + lane; i < pw; i += 32) argmax_combine(v, idx, F::mag2(u1[i]), i);
+#pragma unroll
+        for (int z = 0; z < (PWM + 31) / 32; ++z) {
+          const int i = c + 1 + lane + 32 * z;
+          const double m = F::mag2(u1[min(i, pw - 1)]);
+          if ((i < pw) & (m > v)) {
+            v = m;
+            idx = i;
+          }
+        }
         warp_argmax(v, idx);
         cand = v > 0.0 ? idx : c;
         const double akk2 = F::mag2(akk);
@@ -432,32 +440,32 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     if (q != c + 1) write_col(c + 1, v3);
     __syncthreads();
     if (warp == 0) {
+      constexpr int NZ = (PWM + 31) / 32;  // rows per lane
       int kstep = 1, kp = c;
       bool err = false;
       if (forced) {
         kstep = forced;
         kp = q;
       } else {
-        double rmx = 0.0;
-        for (int i = c + lane; i < pw; i += 32)
-          if (i != q) rmx = fmax(rmx, F::mag2(v2[i]));
+        double rmx = -1.0;
+        int idx = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rmx = fmax(rmx, __shfl_xor_sync(0xffffffffu, rmx, o));
+        for (int z = 0; z < NZ; ++z) {
+          const int i = c + lane + 32 * z;
+          const double m = F::mag2(v2[min(i, pw - 1)]);
+          if ((i < pw) & (i != q) & (m > rmx)) rmx = m;
+        }
+        warp_argmax(rmx, idx);
         const double akk2 = mod_s[0], v = mod_s[1], aqq2 = F::mag2(v2[q]);
         // |a_cc| >= alpha colmax (colmax / rowmax), |a_qq| >= alpha rowmax
         int t1 = quick_ge(akk2 * rmx, alpha * alpha * v * v), t2 = quick_ge(aqq2, alpha * alpha * rmx);
         if (t1 < 0 || (t1 == 0 && t2 < 0)) {
-          const double rowmax = sqrt(rmx), colmax = sqrt(v > 0.0 ? v : 0.0);
+          const double rowmax = sqrt(fmax(rmx, 0.0)), colmax = sqrt(v > 0.0 ? v : 0.0);
           t1 = F::mag(u1[c]) >= alpha * colmax * (colmax / rowmax);
           t2 = F::mag(v2[q]) >= alpha * rowmax;
         }
-        if (t1) {
-        } else if (t2) {
-          kp = q;
-        } else {
-          kstep = 2;
-          kp = q;
-        }
+        kstep = (t1 | t2) ? 1 : 2;
+        kp = t1 ? c : q;
         if (lane == 0 && prec) prec[c] = kstep == 2 ? -kp - 1 : kp;  // (1x1 in place is the default record)
       }
       const int p = kstep == 1 ? c : c + 1;
@@ -468,12 +476,16 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
         T dk = kp == c ? v1c : v2q;
         err = !perturb1(dk, lane == 0);
         const T dinv = panel_recip(dk);
-        for (int i = c + 1 + lane; i < pw; i += 32) {
-          const T o = u1[i];
-          const T u = kp == c ? o : (i == q ? v1q : v2[i]);
-          if (kp != c) rep[i] = i == q ? v1c : o;
-          u1[i] = u;
-          w1[i] = F::mul(u, dinv);
+#pragma unroll
+        for (int z = 0; z < NZ; ++z) {
+          const int i = c + 1 + lane + 32 * z;
+          if (i < pw) {
+            const T o = u1[i], t = v2[i];
+            const T u = sel(kp == c, o, sel(i == q, v1q, t));
+            rep[i] = sel(i == q, v1c, o);
+            u1[i] = u;
+            w1[i] = F::mul(u, dinv);
+          }
         }
         if (lane == 0) w1[c] = dk;
       } else {
@@ -503,16 +515,17 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
         }
         }
         const T detinv = panel_recip(det);
-        for (int i = c + 2 + lane; i < pw; i += 32) {
-          const T x1 = (sw && i == q) ? v1p : u1[i];
-          const T x2 = (sw && i == q) ? v2p : v2[i];
-          const T a1 = F::mul(F::sub(F::mul(d22, x1), F::mul(d21, x2)), detinv);
-          const T a2 = F::mul(F::sub(F::mul(d11, x2), F::mul(d21, x1)), detinv);
-          if (sw) rep[i] = i == q ? v3p : v3[i];
-          u1[i] = x1;
-          u2[i] = x2;
-          w1[i] = a1;
-          w2[i] = a2;
+#pragma unroll
+        for (int z = 0; z < NZ; ++z) {
+          const int i = c + 2 + lane + 32 * z;
+          if (i < pw) {
+            const T x1 = sel(sw && i == q, v1p, u1[i]), x2 = sel(sw && i == q, v2p, v2[i]);
+            rep[i] = sel(i == q, v3p, v3[i]);
+            u1[i] = x1;
+            u2[i] = x2;
+            w1[i] = F::mul(F::sub(F::mul(d22, x1), F::mul(d21, x2)), detinv);
+            w2[i] = F::mul(F::sub(F::mul(d11, x2), F::mul(d21, x1)), detinv);
+          }
         }
         if (lane == 0) {
           w1[c] = a11;
@@ -523,9 +536,6 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
           d_s[c + 1] = d22;
           kd_s[c] = 1;
           kd_s[c + 1] = 2;
-          // the deep rows' inverse is that of the stored D
-          inv_s[c] = pivot_inverse<T>(1, d11, d21, d22);
-          inv_s[c + 1] = F::zero();
           ctl[8] = 1;
         }
       }
@@ -645,10 +655,9 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
 
   // D, kinds and the pivot order
   for (int i = tid; i < pw; i += NT) {
-    if (kd_s[i] == 0) {
-      d_s[i] = Lp[pk_col(i, pw) + i];
-      inv_s[i] = panel_recip(d_s[i]);
-    }
+    if (kd_s[i] == 0) d_s[i] = Lp[pk_col(i, pw) + i];
+    // (the deep rows' inverse of a 2x2 block is that of the stored D)
+    inv_s[i] = pivot_inverse<T>(kd_s[i], d_s[i], ds_s[i], kd_s[i] == 1 ? d_s[i + 1] : F::zero());
     reinterpret_cast<T*>(fa.d)[first + kb + i] = d_s[i];
     reinterpret_cast<T*>(fa.dsub)[first + kb + i] = ds_s[i];
     fa.kind[first + kb + i] = kd_s[i];
@@ -706,8 +715,9 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       __syncthreads();
     }
   }
-  if (fuse && nrow > ke)
-    deep_rows_for<T, PWM / 8, true>(panel, nrow, kb, pw, ke, nrow, Lp, src_s, inv_s, d_s, ds_s, kd_s, ctl[8] != 0);
+  if constexpr (PWM <= GF_MID_PW)  // (no launch with a wider block has fused tasks)
+    if (fuse && nrow > ke)
+      deep_rows_for<T, PWM / 8, true>(panel, nrow, kb, pw, ke, nrow, Lp, src_s, inv_s, d_s, ds_s, kd_s, ctl[8] != 0);
 }
 
 // ---------------------------------------------------------------------------

@@ -715,14 +715,15 @@ void build_plan(rslab_sym_handle& H, const int64_t* col_ptr, const int64_t* row_
       Launch G{L_GETF2, (long long)H.t4.size(), 0, 0};
       std::vector<int4> deep, schur, schur_tc, schur_r, schur_tc_r, narrow;
       int max_pw = 0, max_narrow = 0, max_deep = 0;
-      bool any = false;
+      bool any = false, may_fuse = true;  // (the launch's instance follows its widest block)
+      for (int64_t s : lvl) may_fuse = may_fuse && std::min<int64_t>(nb_of(s), S.sn[s].ncol - (int64_t)b * nb_of(s)) <= FUSE_PW;
       for (int64_t s : lvl) {
         int nb = nb_of(s), nc = (int)S.sn[s].ncol, nr = H.nrow[s];
         int kb = b * nb;
         if (kb >= nc) continue;
         any = true;
         int ke = std::min(kb + nb, nc);
-        bool fuse = (nr - ke) <= FUSE_DEEP_ROWS;
+        bool fuse = (nr - ke) <= FUSE_DEEP_ROWS && may_fuse;
         const bool nar = ke - kb <= GF_NARROW_PW;
         (nar ? narrow : H.t4).push_back(make_int4((int)s, kb, 0, fuse ? 1 : 0));
         (nar ? max_narrow : max_pw) = std::max(nar ? max_narrow : max_pw, ke - kb);
@@ -2879,12 +2880,12 @@ int noalloc_count(int nrow, int ncol, int nb, std::vector<NoallocSeg>& segs) {
   int t = 0;
   for (int kb = 0; kb < ncol; kb += nb) {
     const int ke = std::min(kb + nb, ncol);
-    const bool fuse = (nrow - ke) <= NOALLOC_FUSE_ROWS;
+    const bool fuse = (nrow - ke) <= NOALLOC_FUSE_ROWS && nb <= FUSE_PW;
     segs.push_back({L_GETF2, t, 1});
     t += 1;
     if (!fuse) {
       const int cnt = (nrow - ke + DEEP_R - 1) / DEEP_R;
-      segs.push_back({L_DEEP, t, cnt});
+      if (cnt) segs.push_back({L_DEEP, t, cnt});
       t += cnt;
     }
     const int cnt = noalloc_schur_tiles(nrow - ke, ncol - ke);
@@ -2908,7 +2909,7 @@ __global__ void k_noalloc_plan(NoallocStruct* ns, int4* tasks, int nrow, int nco
   int t = 0;
   for (int kb = 0; kb < ncol; kb += nb) {
     const int ke = min(kb + nb, ncol);
-    const bool fuse = (nrow - ke) <= NOALLOC_FUSE_ROWS;
+    const bool fuse = (nrow - ke) <= NOALLOC_FUSE_ROWS && nb <= FUSE_PW;
     if (threadIdx.x == 0) tasks[t] = make_int4(0, kb, 0, fuse ? 1 : 0);
     t += 1;
     if (!fuse) {

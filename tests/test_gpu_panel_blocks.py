@@ -28,7 +28,7 @@ def dense_lower(n, dtype, dominant, seed):
 @pytest.mark.parametrize("dtype", [np.float64, np.complex128, np.float32, np.complex64])
 @pytest.mark.parametrize("n,nb", [(1, 64), (2, 64), (8, 64), (9, 64), (31, 64), (32, 64), (33, 64), (63, 64), (64, 64),
                                   (65, 64), (97, 64), (128, 64), (129, 64), (193, 64), (150, 17), (200, 128),
-                                  (513, 64), (600, 8)])
+                                  (513, 64), (600, 8), (576, 64), (640, 64)])
 def test_dense_panel_is_the_oracles(n, nb, dtype):
     for dominant in (False, True):
         a = dense_lower(n, dtype, dominant, n + nb)
@@ -40,3 +40,35 @@ def test_dense_panel_is_the_oracles(n, nb, dtype):
         assert np.array_equal(g.perm, o.perm)
         assert np.array_equal(g.d_diag, o.d_diag) and np.array_equal(g.d_subdiag, o.d_subdiag)
         assert np.array_equal(g.l_row_idx, o.l_row_idx) and np.array_equal(g.l_values, o.l_values)
+
+
+def test_wide_and_narrow_supernodes_of_one_level():
+    """Blocks of 128, 64 and a few columns in the same launches, with few and
+    many deep rows: leaves of one parent, in one matrix."""
+    rng = np.random.default_rng(5)
+    widths, sep = (600, 90, 40, 64, 5), 70
+    n = sum(widths) + sep
+    full = np.zeros((n, n))
+    at = 0
+    for w in widths:
+        full[at:at + w, at:at + w] = rng.standard_normal((w, w))
+        full[n - sep:, at:at + w] = rng.standard_normal((sep, w))
+        at += w
+    full[n - sep:, n - sep:] = rng.standard_normal((sep, sep))
+    full = np.tril(full)
+    r, c = np.nonzero(full)
+    a = CscMatrix.from_triplets(n, r, c, full[r, c])
+    for engine in ("fma", "tensor"):
+        st = SolverSettings(ordering=Ordering.NATURAL, schur_engine=engine)
+        sym = LdltSymbolic.analyze_with(a, st)
+        g = sym.factor(a, st)
+        o = OracleSolver(a, sym.export())
+        b = rng.standard_normal(n)
+        if engine == "fma":
+            f, e = g.export_factors(), o.factors()
+            assert np.array_equal(f.perm, e.perm) and np.array_equal(f.l_values, e.l_values)
+        A = a.to_scipy_full()
+        x, xo = g.solve(b), o.solve_many(b.reshape(n, 1), 1).reshape(n)
+        scale = abs(A).sum(axis=1).max()
+        be = [float(np.max(np.abs(b - A @ v)) / (scale * np.max(np.abs(v)) + np.max(np.abs(b)))) for v in (x, xo)]
+        assert be[0] <= max(1e-13, 10 * be[1])
