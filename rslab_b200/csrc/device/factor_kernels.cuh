@@ -258,8 +258,8 @@ __device__ __forceinline__ int lower_bound_i(const int* __restrict__ a, int lo, 
 // Per pair the product U = L_k[a.., :] G_k[q0.., :]^T (G_k = L21_k D_k,
 // formed once per updater by k_make_g with ld_G's arithmetic) runs in the
 // updater's row space: operands are contiguous column runs of k's panel and
-// of G_k, staged by cp.async into two shared-memory stages (the next chunk,
-// possibly of the next pair, loads while the current one is multiplied).
+// of G_k, staged by cp.async in shared memory (the next chunks, possibly of
+// the next pairs, load while the current one is multiplied).
 // 128 threads, warp w owns rows 16w..16w+15 of the pair, each thread an 8 x 4
 // register micro-tile (8 consecutive rows, columns cx + 16 j: conflict-free
 // shared-memory reads); warps whose rows lie past nr skip the arithmetic.
@@ -267,31 +267,54 @@ __device__ __forceinline__ int lower_bound_i(const int* __restrict__ a, int lo, 
 // subtracted from the tile held in shared memory through the pair's row /
 // column maps (rows r >= column c in k's ordering only): the same operations
 // in the same order as the oracle, so the result is bit-identical to it.
+//
+// This engine runs the small factors, where a tile has tens of pairs of a few
+// columns each: bound by the latency of a pair, not by its arithmetic.  So
+// the descriptors of CM_PB pairs are fetched together (their panel offsets
+// hang off two dependent loads), and CM_STAGES operand chunks, with the pairs'
+// row indices, are in flight by cp.async; and a pair of at most CM_SMALL
+// outputs (most of a 2D grid's) is formed one output per thread: the micro-tile
+// would run 32 products a column for a handful, and 32 scatter tests.
+// 480-unknown 2D grid: 0.264 ms in five launches with descriptors read per
+// pair, one chunk ahead and micro-tiles only (0.253 with the first two alone),
+// 0.150 now; a KKT factor of 1,866 unknowns 0.407 -> 0.325.
 // ---------------------------------------------------------------------------
 constexpr int CM_NT = 128;
-template <typename T> struct CmChunk { static constexpr int v = 16; };
-template <> struct CmChunk<c64> { static constexpr int v = 8; };
+constexpr int CM_PB = 32;  // pair descriptors per shared-memory batch
+constexpr int CM_SMALL = 4 * CM_NT;  // outputs of a pair up to which every thread owns single outputs
+template <typename T> struct CmChunk { static constexpr int v = 16, stages = 4; };
+template <> struct CmChunk<c64> { static constexpr int v = 8, stages = 2; };  // two CTAs per SM
 
-// Shared memory of k_cmod: the tile, two operand stages, two row / column
-// maps and the tile's row structure.
+struct CmPair {
+  long long a_off, b_off, r_off;  // L21 rows of the pair, G rows, first off-diagonal row index
+  int lda, ldb, nck, a, q0, nr, nc;
+};
+
+// Shared memory of k_cmod: the tile, the operand stages with their row and
+// column indices, the row / column maps, the tile's row structure and the
+// pair descriptors.
 template <typename T>
 __host__ __device__ constexpr size_t smem_cmod_bytes() {
-  return (size_t)TILE * TILE * sizeof(T) + 2 * 2 * (size_t)CmChunk<T>::v * TILE * sizeof(T) + 5 * TILE * 4 + 16;
+  return (size_t)TILE * TILE * sizeof(T) +
+         CmChunk<T>::stages * (2 * (size_t)CmChunk<T>::v * TILE * sizeof(T) + 2 * TILE * 4) + 3 * TILE * 4 +
+         CM_PB * sizeof(CmPair) + 16;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(CM_NT, 2) k_cmod(FactorArgs fa, const int4* __restrict__ tasks,
                                                    const int4* __restrict__ pairs) {
   using F = Field<T>;
-  constexpr int KC = CmChunk<T>::v;
+  constexpr int KC = CmChunk<T>::v, NST = CmChunk<T>::stages;
   constexpr int STAGE = 2 * KC * TILE;  // A chunk [t][64 rows] then B chunk [t][64 cols]
   if (fa.status[0] != 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* acc_s = reinterpret_cast<T*>(smem_raw);  // [64 cols][64 rows]
-  T* stg = acc_s + TILE * TILE;               // 2 stages
-  int* rs_tile = reinterpret_cast<int*>(stg + 2 * STAGE);  // 64
-  int* rowmap = rs_tile + TILE;                            // 2 x 64 (pair parity)
-  int* colmap = rowmap + 2 * TILE;                         // 2 x 64
+  T* stg = acc_s + TILE * TILE;               // NST stages
+  CmPair* prs = reinterpret_cast<CmPair*>(stg + NST * STAGE);
+  int* ids = reinterpret_cast<int*>(prs + CM_PB);  // per stage: 64 row and 64 column indices
+  int* rs_tile = ids + NST * 2 * TILE;             // 64
+  int* rowmap = rs_tile + TILE;                    // 64
+  int* colmap = rowmap + TILE;                     // 64
 
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, r0 = (tk.y >> 16) * TILE, c0 = (tk.y & 0xffff) * TILE;
@@ -310,31 +333,37 @@ __global__ void __launch_bounds__(CM_NT, 2) k_cmod(FactorArgs fa, const int4* __
   const T* pall = reinterpret_cast<const T*>(fa.panel);
   const T* gall = reinterpret_cast<const T*>(fa.gpool);
 
-  // chunk stream over (pair u, columns [t0, t0 + KC) of its updater)
+  // chunk stream over (pair u of the batch, columns [t0, t0 + KC) of its updater)
   struct Cur {
     int u, t0;
   };
   auto issue = [&](Cur x, int st) {
-    const int4 pr = pairs[x.u];
-    const int k = pr.x, a = pr.y, q0 = pr.z, nr = pr.w >> 16, nc = pr.w & 0xffff;
-    const int nck = fa.sn_ncol[k], nrk = fa.sn_nrow[k];
-    const T* A = pall + fa.sn_poff[k] + nck + a;
-    const T* B = gall + fa.goff[k] + q0;
-    const long long ldb = nrk - nck;
+    const CmPair& p = prs[x.u];
+    const T* A = pall + p.a_off;
+    const T* B = gall + p.b_off;
     T* As = stg + st * STAGE;
     T* Bs = As + KC * TILE;
-    for (int e = tid; e < KC * TILE; e += CM_NT) {
-      const int t = e / TILE, r = e % TILE, tt = x.t0 + t;
-      const bool in_t = tt < nck;
-      cp_async_zfill<(int)sizeof(T)>(As + e, in_t && r < nr ? A + r + (long long)tt * nrk : A, in_t && r < nr);
-      cp_async_zfill<(int)sizeof(T)>(Bs + e, in_t && r < nc ? B + r + (long long)tt * ldb : B, in_t && r < nc);
+    const int nr = p.nr, nc = p.nc, kt = p.nck - x.t0;
+    const int r = tid % TILE, tb = tid / TILE;
+    const T* Ar = A + r + (long long)(x.t0 + tb) * p.lda;
+    const T* Br = B + r + (long long)(x.t0 + tb) * p.ldb;
+    const long long sa = (CM_NT / TILE) * (long long)p.lda, sb = (CM_NT / TILE) * (long long)p.ldb;
+#pragma unroll
+    for (int q = 0; q < KC * TILE / CM_NT; ++q) {
+      const bool in_t = tb + q * (CM_NT / TILE) < kt;
+      const int e = tid + q * CM_NT;
+      cp_async_zfill<(int)sizeof(T)>(As + e, in_t && r < nr ? Ar + q * sa : A, in_t && r < nr);
+      cp_async_zfill<(int)sizeof(T)>(Bs + e, in_t && r < nc ? Br + q * sb : B, in_t && r < nc);
     }
-    cp_async_commit();
+    if (x.t0 == 0) {
+      const int* ok = fa.rs + p.r_off + (tid < TILE ? p.a : p.q0);
+      const int i = tid & (TILE - 1);
+      if (i < (tid < TILE ? nr : nc)) cp_async_zfill<4>(ids + st * 2 * TILE + tid, ok + i, true);
+    }
   };
   auto advance = [&](Cur x) -> Cur {
-    const int nck = fa.sn_ncol[pairs[x.u].x];
     x.t0 += KC;
-    if (x.t0 >= nck) {
+    if (x.t0 >= prs[x.u].nck) {
       x.u += 1;
       x.t0 = 0;
     }
@@ -349,79 +378,123 @@ __global__ void __launch_bounds__(CM_NT, 2) k_cmod(FactorArgs fa, const int4* __
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = F::zero();
 
-  Cur cur{tk.z, 0};
-  if (tk.z < tk.w) issue(cur, 0);
-  int st = 0, parity = 0;
-  while (cur.u < tk.w) {
-    const int4 pr = pairs[cur.u];
-    const int k = pr.x, a = pr.y, q0 = pr.z, nr = pr.w >> 16, nc = pr.w & 0xffff;
-    const int nck = fa.sn_ncol[k];
-    if (cur.t0 == 0) {
-      // the tile positions of this pair's rows and columns (read only at the
-      // pair's scatter, after at least one block barrier)
-      __syncthreads();  // rs_tile written / the map slot's previous reader done
-      const int* ok = fa.rs + fa.sn_rsoff[k] + nck;
-      if (tid < nr) rowmap[parity * TILE + tid] = lower_bound_i(rs_tile, 0, rows_here, ok[a + tid]);
-      if (tid >= TILE && tid - TILE < nc) colmap[parity * TILE + tid - TILE] = ok[q0 + tid - TILE] - first - c0;
-    }
-    const Cur nx = advance(cur);
-    if (nx.u < tk.w) {
-      issue(nx, st ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+  for (int u0 = tk.z; u0 < tk.w; u0 += CM_PB) {
+    const int np = min(CM_PB, tk.w - u0);
+    __syncthreads();  // the previous batch's descriptors and stages are free (first: the tile is written)
+    for (int e = tid; e < np; e += CM_NT) {
+      const int4 pr = pairs[u0 + e];
+      const int k = pr.x, nck = fa.sn_ncol[k], nrk = fa.sn_nrow[k];
+      prs[e] = CmPair{fa.sn_poff[k] + nck + pr.y, fa.goff[k] + pr.z, fa.sn_rsoff[k] + nck, nrk, nrk - nck, nck,
+                      pr.y, pr.z, pr.w >> 16, pr.w & 0xffff};
     }
     __syncthreads();
-    const T* As = stg + st * STAGE;
-    const T* Bs = As + KC * TILE;
-    const int kt = min(KC, nck - cur.t0);
-    if (rb - 8 * ry < nr) {  // the warp has rows of this pair
-      if (kt == KC) {
-#pragma unroll 2
-        for (int t = 0; t < KC; ++t) {
-          T av[8], bv[4];
-          lds_row<T, 8>(As + t * TILE + rb, av);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) bv[j] = Bs[t * TILE + cx + 16 * j];
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = F::fma_(av[i], bv[j], acc[i][j]);
-        }
-      } else {
-        for (int t = 0; t < kt; ++t) {
-          T av[8], bv[4];
-          lds_row<T, 8>(As + t * TILE + rb, av);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) bv[j] = Bs[t * TILE + cx + 16 * j];
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = F::fma_(av[i], bv[j], acc[i][j]);
-        }
+    Cur cur{0, 0}, nxt{0, 0};
+    int si = 0, sc = 0;  // issue / compute stage
+#pragma unroll 1
+    for (int q = 0; q < NST - 1; ++q) {
+      if (nxt.u < np) {
+        issue(nxt, si);
+        nxt = advance(nxt);
+        si = si + 1 == NST ? 0 : si + 1;
       }
+      cp_async_commit();
     }
-    if (nx.u != cur.u) {
-      // the pair is complete: subtract it from the tile, reset the registers
+    while (cur.u < np) {
+      if (nxt.u < np) {
+        issue(nxt, si);
+        nxt = advance(nxt);
+        si = si + 1 == NST ? 0 : si + 1;
+      }
+      cp_async_commit();
+      cp_async_wait<NST - 1>();
+      __syncthreads();  // the chunk landed everywhere; the last pair's scatter is done
+      const CmPair& p = prs[cur.u];
+      const int nr = p.nr, nc = p.nc, a = p.a, q0 = p.q0;
+      if (cur.t0 == 0) {
+        // the tile positions of this pair's rows and columns (read at the
+        // pair's scatter, after the next barrier)
+        const int* id = ids + sc * 2 * TILE;
+        if (tid < nr) rowmap[tid] = lower_bound_i(rs_tile, 0, rows_here, id[tid]);
+        if (tid >= TILE && tid - TILE < nc) colmap[tid - TILE] = id[tid] - first - c0;
+      }
+      const T* As = stg + sc * STAGE;
+      const T* Bs = As + KC * TILE;
+      const int kt = min(KC, p.nck - cur.t0);
+      // a pair of at most CM_SMALL outputs: one output per thread and pass
+      // instead of a mostly empty micro-tile (its results in acc[0][.])
+      const bool small = nr * nc <= CM_SMALL;
+      if (small) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int ri = rb + i;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int cj = cx + 16 * j;
-          if (ri < nr && cj < nc && a + ri >= q0 + cj) {
-            const int e = colmap[parity * TILE + cj] * TILE + rowmap[parity * TILE + ri];
-            acc_s[e] = F::sub(acc_s[e], acc[i][j]);
+        for (int z = 0; z < CM_SMALL / CM_NT; ++z) {
+          const int o = tid + z * CM_NT;
+          if (o < nr * nc) {
+            const int cj = o / nr, ri = o - cj * nr;
+            T v = acc[0][z];
+#pragma unroll 4
+            for (int t = 0; t < kt; ++t) v = F::fma_(As[t * TILE + ri], Bs[t * TILE + cj], v);
+            acc[0][z] = v;
           }
-          acc[i][j] = F::zero();
+        }
+      } else if (rb - 8 * ry < nr) {  // the warp has rows of this pair
+        if (kt == KC) {
+#pragma unroll 2
+          for (int t = 0; t < KC; ++t) {
+            T av[8], bv[4];
+            lds_row<T, 8>(As + t * TILE + rb, av);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bv[j] = Bs[t * TILE + cx + 16 * j];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) acc[i][j] = F::fma_(av[i], bv[j], acc[i][j]);
+          }
+        } else {
+          for (int t = 0; t < kt; ++t) {
+            T av[8], bv[4];
+            lds_row<T, 8>(As + t * TILE + rb, av);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bv[j] = Bs[t * TILE + cx + 16 * j];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) acc[i][j] = F::fma_(av[i], bv[j], acc[i][j]);
+          }
         }
       }
-      parity ^= 1;
+      const Cur after = advance(cur);
+      __syncthreads();  // the stage is free for the next issue; the maps are written
+      if (after.u != cur.u && small) {
+#pragma unroll
+        for (int z = 0; z < CM_SMALL / CM_NT; ++z) {
+          const int o = tid + z * CM_NT;
+          const int cj = o / nr, ri = o - cj * nr;
+          if (o < nr * nc && a + ri >= q0 + cj) {
+            const int e = colmap[cj] * TILE + rowmap[ri];
+            acc_s[e] = F::sub(acc_s[e], acc[0][z]);
+          }
+          acc[0][z] = F::zero();
+        }
+      } else if (after.u != cur.u) {
+        // the pair is complete: subtract it from the tile, reset the registers
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int ri = rb + i;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int cj = cx + 16 * j;
+            if (ri < nr && cj < nc && a + ri >= q0 + cj) {
+              const int e = colmap[cj] * TILE + rowmap[ri];
+              acc_s[e] = F::sub(acc_s[e], acc[i][j]);
+            }
+            acc[i][j] = F::zero();
+          }
+        }
+      }
+      sc = sc + 1 == NST ? 0 : sc + 1;
+      cur = after;
     }
-    __syncthreads();  // the stage is free for the load after next
-    st ^= 1;
-    cur = nx;
   }
+  cp_async_wait<0>();
   __syncthreads();
   for (int e = tid; e < TILE * TILE; e += CM_NT) {
     const int c = e / TILE, r = e % TILE;
