@@ -20,8 +20,11 @@
 // an interchange or a 2x2 pivot) have the candidate column and column k + 1
 // written to shared memory, warp 0 composes the post-interchange columns, and
 // the owners of the interchanged row and column reload them.  Every entry
-// sees the operations of the reference in its order, so the factor is the
-// oracle's bit for bit in every field.
+// sees the operations of the reference in its order, so with EXACT (the FMA
+// engine) the factor is the oracle's bit for bit in every field; the tensor
+// engine, whose products are summed in tiles anyway, takes fused updates and
+// one division per complex reciprocal, except in real f64 (64-column block
+// with either form: c32 44 / 32 us, 128 columns of c64 104 / 75, f64 31 / 28).
 // The finished columns collect in shared memory (packed lower triangle).
 // Measured (B200): a diagonally dominant 64-column block on one CTA takes 31
 // us in f64 and 42 us in c32 (0.35 and 0.5 us a step); a shared-memory block
@@ -118,6 +121,28 @@ __device__ __forceinline__ cplx<R> panel_recip(cplx<R> a) {
   return Field<cplx<R>>::recip(a);
 }
 
+// e - u w: the reference's multiply and subtract, each rounded (zero
+// multipliers skipped, as there), or fused.
+template <typename T, bool EXACT>
+__device__ __forceinline__ T minus_prod(T e, T u, T w) {
+  using F = Field<T>;
+  if constexpr (EXACT)
+    return sel(F::is_zero(w), e, F::sub(e, F::mul(u, w)));
+  else
+    return F::fnma(u, w, e);
+}
+// 1 / a for the multipliers: the reference's two divisions of a complex
+// reciprocal, or one reciprocal of |a|^2.
+template <typename T, bool EXACT>
+__device__ __forceinline__ T step_recip(T a) {
+  if constexpr (EXACT || !Field<T>::complex) {
+    return panel_recip(a);
+  } else {
+    const auto r = panel_recip(quick2(a));
+    return T{a.re * r, -a.im * r};
+  }
+}
+
 // Inverse of the pivot block that starts at position k (1x1: 1 / d; 2x2:
 // 1 / (d11 d22 - d21^2); zero for the second position of a 2x2).
 template <typename T>
@@ -163,12 +188,7 @@ __device__ __forceinline__ void deep_rows(T* panel, long long nrow, int kb, int 
         for (int s = s0; s < NSL; ++s) {
           const T l0 = Lk[8 * s];
           const T l = s > s0 ? l0 : sel(t > t0, l0, F::zero());
-          if constexpr (EXACT) {
-            const T v = F::sub(x[s], F::mul(xk, l));
-            x[s] = sel(F::is_zero(l), x[s], v);
-          } else {
-            x[s] = F::fnma(xk, l, x[s]);
-          }
+          x[s] = minus_prod<T, EXACT>(x[s], xk, l);
         }
       }
     }
@@ -219,7 +239,7 @@ __device__ __forceinline__ void deep_rows_for(T* panel, long long nrow, int kb, 
 // ---------------------------------------------------------------------------
 // getf2: task (s, kb, -, fuse).
 // ---------------------------------------------------------------------------
-template <typename T, int G, int NS>
+template <typename T, int G, int NS, bool EXACT>
 __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     k_getf2(FactorArgs fa, const int4* __restrict__ tasks, int nb_small, int nb_big) {
   using F = Field<T>;
@@ -324,7 +344,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     const int cx = c - off;
     const T akk = shfl_t(a[0], (cx * G + cx) & 31);
     const R akk2 = quick2(akk);
-    const T dinv = panel_recip(akk);
+    const T dinv = step_recip<T, EXACT>(akk);
     const int rem = pw - c, lc = pk_col(c, pw);
     bool doubt = !((akk2 >= lo2) & (akk2 <= Q::hi));
     if (reuse) doubt = doubt | (rec_s[c] != c);
@@ -595,9 +615,10 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
 #pragma unroll
           for (int jj = 0; jj < NS; ++jj)
             if (jj <= ii) {
-              const T e = a[ix(ii, jj)], w = w1[off + tx + G * jj], v = F::sub(e, F::mul(x, w));
-              const T vb = F::sub(v, F::mul(x2, w2[off + tx + G * jj]));
-              a[ix(ii, jj)] = sel(kstep == 2, vb, sel(F::is_zero(w), e, v));
+              const T e = a[ix(ii, jj)], w = w1[off + tx + G * jj], wb = w2[off + tx + G * jj];
+              const T vb = EXACT ? F::sub(F::sub(e, F::mul(x, w)), F::mul(x2, wb)) : F::fnma(x2, wb, F::fnma(x, w, e));
+              const T v = minus_prod<T, EXACT>(e, x, w);
+              a[ix(ii, jj)] = sel(kstep == 2, vb, v);
             }
         }
     }
@@ -622,8 +643,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
         wc[ii] = w1[G * ii];
       }
       auto upd = [&](int ii, int jj) __attribute__((always_inline)) {
-        const T e = a[ix(ii, jj)];
-        a[ix(ii, jj)] = sel(F::is_zero(wc[jj]), e, F::sub(e, F::mul(ur[ii], wc[jj])));
+        a[ix(ii, jj)] = minus_prod<T, EXACT>(a[ix(ii, jj)], ur[ii], wc[jj]);
       };
       // the columns beyond slot column 0 (rows past the block are skipped
       // where that saves more than the branch)
@@ -717,7 +737,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
   }
   if constexpr (PWM <= GF_MID_PW)  // (no launch with a wider block has fused tasks)
     if (fuse && nrow > ke)
-      deep_rows_for<T, PWM / 8, true>(panel, nrow, kb, pw, ke, nrow, Lp, src_s, inv_s, d_s, ds_s, kd_s, ctl[8] != 0);
+      deep_rows_for<T, PWM / 8, EXACT>(panel, nrow, kb, pw, ke, nrow, Lp, src_s, inv_s, d_s, ds_s, kd_s, ctl[8] != 0);
 }
 
 // ---------------------------------------------------------------------------

@@ -958,15 +958,15 @@ size_t smem_diag_inv(size_t es) { return (size_t)TB * (TB + 1) * 2 * es; }
 // The panel kernels of a launch whose widest block has `pw` columns: the
 // smallest k_getf2 instance (64 threads up to 32 columns, 256 above) and the
 // smallest k_deep one (8 columns per slot) that hold it.
-template <typename T>
+template <typename T, bool EXACT>
 void launch_getf2(int pw, int ntasks, cudaStream_t st, const FactorArgs& fa, const int4* tasks, int nb_small,
                   int nb_big) {
   if (pw <= GF_NARROW_PW)
-    k_getf2<T, GF_NARROW_G, 4><<<ntasks, 64, smem_getf2(sizeof(T), GF_NARROW_PW), st>>>(fa, tasks, nb_small, nb_big);
+    k_getf2<T, GF_NARROW_G, 4, EXACT><<<ntasks, 64, smem_getf2(sizeof(T), GF_NARROW_PW), st>>>(fa, tasks, nb_small, nb_big);
   else if (pw <= GF_MID_PW)
-    k_getf2<T, GF_G, 4><<<ntasks, 256, smem_getf2(sizeof(T), GF_MID_PW), st>>>(fa, tasks, nb_small, nb_big);
+    k_getf2<T, GF_G, 4, EXACT><<<ntasks, 256, smem_getf2(sizeof(T), GF_MID_PW), st>>>(fa, tasks, nb_small, nb_big);
   else
-    k_getf2<T, GF_G, 8><<<ntasks, 256, smem_getf2(sizeof(T), GF_WIDE_PW), st>>>(fa, tasks, nb_small, nb_big);
+    k_getf2<T, GF_G, 8, EXACT><<<ntasks, 256, smem_getf2(sizeof(T), GF_WIDE_PW), st>>>(fa, tasks, nb_small, nb_big);
 }
 template <typename T, bool EXACT>
 void launch_deep(int pw, int ntasks, cudaStream_t st, const FactorArgs& fa, const int4* tasks, int nb_small,
@@ -977,17 +977,22 @@ void launch_deep(int pw, int ntasks, cudaStream_t st, const FactorArgs& fa, cons
     k_deep<T, 16, EXACT><<<ntasks, DEEP_NT, smem_deep(sizeof(T), GF_WIDE_PW), st>>>(fa, tasks, nb_small, nb_big);
 }
 // Their shared-memory limits (once per device).
-template <typename T>
-void panel_attrs() {
+template <typename T, bool EXACT>
+void panel_attrs_of() {
   const size_t es = sizeof(T);
   constexpr auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  CK(cudaFuncSetAttribute(k_getf2<T, GF_NARROW_G, 4>, A, (int)smem_getf2(es, GF_NARROW_PW)));
-  CK(cudaFuncSetAttribute(k_getf2<T, GF_G, 4>, A, (int)smem_getf2(es, GF_MID_PW)));
-  CK(cudaFuncSetAttribute(k_getf2<T, GF_G, 8>, A, (int)smem_getf2(es, GF_WIDE_PW)));
-  CK(cudaFuncSetAttribute(k_deep<T, 8, true>, A, (int)smem_deep(es, GF_MID_PW)));
-  CK(cudaFuncSetAttribute(k_deep<T, 16, true>, A, (int)smem_deep(es, GF_WIDE_PW)));
-  CK(cudaFuncSetAttribute(k_deep<T, 8, false>, A, (int)smem_deep(es, GF_MID_PW)));
-  CK(cudaFuncSetAttribute(k_deep<T, 16, false>, A, (int)smem_deep(es, GF_WIDE_PW)));
+  if constexpr (EXACT || !std::is_same_v<T, double>) {
+    CK(cudaFuncSetAttribute(k_getf2<T, GF_NARROW_G, 4, EXACT>, A, (int)smem_getf2(es, GF_NARROW_PW)));
+    CK(cudaFuncSetAttribute(k_getf2<T, GF_G, 4, EXACT>, A, (int)smem_getf2(es, GF_MID_PW)));
+    CK(cudaFuncSetAttribute(k_getf2<T, GF_G, 8, EXACT>, A, (int)smem_getf2(es, GF_WIDE_PW)));
+  }
+  CK(cudaFuncSetAttribute(k_deep<T, 8, EXACT>, A, (int)smem_deep(es, GF_MID_PW)));
+  CK(cudaFuncSetAttribute(k_deep<T, 16, EXACT>, A, (int)smem_deep(es, GF_WIDE_PW)));
+}
+template <typename T>
+void panel_attrs() {
+  panel_attrs_of<T, true>();
+  panel_attrs_of<T, false>();
 }
 
 // Fields whose descendant updates can run on the tf32 tensor cores.
@@ -1364,9 +1369,16 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
                                                                  H.d_linv_off);
         break;
       case L_GETF2:
-        launch_getf2<T>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
+        // the FMA engine in the oracle's operation order, the tensor engine
+        // fused, except real f64: a near-singular KKT fixture flips the sign of
+        // a pivot with fused updates (which would save 10% there, against 20-30%
+        // in the complex fields)
+        if (mm)
+          launch_getf2<T, std::is_same_v<T, double>>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
+        else
+          launch_getf2<T, true>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
         break;
-      case L_DEEP:  // the FMA engine in the oracle's operation order, the tensor engine fused
+      case L_DEEP:  // (the same rule, fused in every field of the tensor engine)
         if (mm)
           launch_deep<T, false>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
         else
@@ -2979,7 +2991,7 @@ void noalloc_panel(unsigned char* base, T* panel, int nrow, int ncol, int panel_
   const int4* dt = reinterpret_cast<const int4*>(base + off_tasks);
   for (const NoallocSeg& g : segs) {
     if (g.kind == L_GETF2)
-      launch_getf2<T>(std::min(nb, ncol), g.cnt, st, fa, dt + g.off, nb_small, nb_big);
+      launch_getf2<T, true>(std::min(nb, ncol), g.cnt, st, fa, dt + g.off, nb_small, nb_big);
     else if (g.kind == L_DEEP)
       launch_deep<T, true>(std::min(nb, ncol), g.cnt, st, fa, dt + g.off, nb_small, nb_big);
     else
