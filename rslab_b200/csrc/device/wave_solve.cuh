@@ -63,26 +63,36 @@ constexpr int CH_GROUPS = RHS_MAX / CH_NR;
 // blocks in a level from which its chains take every column of a pass
 constexpr int CH_WIDE_ITEMS = 600;
 
-// Stages in flight: 4, or 3 where the wide elements of 16 right-hand sides
-// would otherwise keep a second CTA off the SM.
+// Stages: 4, three for 16-byte elements, two for 16 columns of the smaller ones
+// (the next unit loads while one is multiplied).
 template <typename T>
 __host__ __device__ constexpr int st_stages(int nr) {
-  return (sizeof(T) >= 16 || (sizeof(T) >= 8 && nr >= 16)) ? 3 : 4;
+  return sizeof(T) >= 16 ? 3 : nr >= 16 ? 2 : 4;
 }
+// Columns whose slice partials are exchanged at a time, and the CTAs per SM the
+// kernel is compiled for.  Sixteen columns of 4- and 8-byte elements: two
+// stages and partials by halves, three CTAs per SM instead of two (64^3 mixed
+// step 54.9 -> 52.6 ms).  The same for c64 (two CTAs instead of one, 128
+// registers) was 0.7% slower, so c64 keeps one.
+template <typename T>
+__host__ __device__ constexpr int st_red_cols(int nr) {
+  return nr < 16 || sizeof(T) >= 16 ? nr : 8;
+}
+__host__ __device__ constexpr int st_minb(size_t es, int nr) { return nr < 16 ? 3 : es >= 16 ? 1 : 3; }
 
 // Right-hand-side buffers are sized by the pass's column count nr (<=
 // RHS_MAX), so a one-column solve keeps several CTAs resident per SM; the
 // kernels are instantiated for NR = 1, 4 and 16 register columns (the
 // smallest NR >= nr runs) so the inner loops carry no dead columns.
 // Streaming: stages of (tile + 32 x nr right-hand sides), then the slice
-// partials (4 x nr x 65).
+// partials (4 x st_red_cols x 65).
 template <typename T>
 __host__ __device__ constexpr size_t st_stage_elems(int nr) {
   return (size_t)ST_UNIT + 32 * nr;
 }
 template <typename T>
 __host__ __device__ constexpr size_t st_smem_bytes(int nr) {
-  return ((size_t)st_stages<T>(nr) * st_stage_elems<T>(nr) + 4 * 65 * nr) * sizeof(T) + 16;
+  return ((size_t)st_stages<T>(nr) * st_stage_elems<T>(nr) + 4 * 65 * st_red_cols<T>(nr)) * sizeof(T) + 16;
 }
 // Chain: one tile slot (its copy overlaps the wait for the dependency's
 // flag; after the chain it holds the slice partials), the inverse block,
@@ -264,14 +274,14 @@ __device__ __forceinline__ void st_issue(T* S, T* Vs, const StItem<T, FWD>& it, 
 }
 
 template <typename T, bool FWD, int NR>
-__global__ void __launch_bounds__(WV_NT) k_stream(SolveArgs a, const int4* __restrict__ tasks) {
+__global__ void __launch_bounds__(WV_NT, st_minb(sizeof(T), NR)) k_stream(SolveArgs a, const int4* __restrict__ tasks) {
   using F = Field<T>;
-  constexpr int NST = st_stages<T>(NR);
+  constexpr int NST = st_stages<T>(NR), RC = st_red_cols<T>(NR);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nr = a.nrhs, ld = a.ld;
   constexpr int SE = (int)st_stage_elems<T>(NR);
   T* stages = reinterpret_cast<T*>(smem_raw);  // NST x (tile, V rows of stride NR)
-  T* red = stages + NST * SE;                  // slice partials, 4 x NR x 65
+  T* red = stages + NST * SE;                  // slice partials, 4 x RC x 65
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x;
   const StItem<T, FWD> it = st_item<T, FWD>(a, tk);
@@ -281,34 +291,37 @@ __global__ void __launch_bounds__(WV_NT) k_stream(SolveArgs a, const int4* __res
   for (int c = 0; c < NR; ++c) acc[c] = F::zero();
   // slice partials of the finished output block -> U (forward) / Wb / slot
   auto flush = [&](int rb) {
-    store_partials<T, NR>(red, acc, x, g);
 #pragma unroll
-    for (int c = 0; c < NR; ++c) acc[c] = F::zero();
-    __syncthreads();
-    for (int e = tid; e < 64 * nr; e += WV_NT) {
-      const int r = e / nr, c = e - r * nr;
-      const T v = slice_sum<T, NR>(red, r, c);
-      if (FWD) {
-        const int row = it.r0 + 64 * rb + r;
-        if (row < it.rlim) {
-          if (tk.w < 0) {
-            T* Us = reinterpret_cast<T*>(a.U) + a.c0 + a.uoff[s] * ld;
-            Us[(long long)(row - a.sn_ncol[s]) * ld + c] = v;
-          } else {
-            T* part = reinterpret_cast<T*>(a.Wp) + (long long)tk.w * 64 * ld;
-            part[(long long)r * ld + c] = v;
-          }
+    for (int h = 0; h < NR; h += RC) {
+      if (h > 0) {
+        if (h >= nr) break;
+        __syncthreads();  // the columns before are summed
+      }
+#pragma unroll
+      for (int c = 0; c < RC; ++c) red[(g * RC + c) * 65 + x] = acc[h + c];
+      __syncthreads();
+      const int nc = min(RC, nr - h);
+      for (int e = tid; e < 64 * nc; e += WV_NT) {
+        const int r = e / nc, c = e - r * nc;
+        const T v = slice_sum<T, RC>(red, r, c);
+        T* out = nullptr;
+        if (FWD) {
+          const int row = it.r0 + 64 * rb + r;
+          if (row < it.rlim && tk.w < 0)
+            out = reinterpret_cast<T*>(a.U) + a.c0 + (a.uoff[s] + row - a.sn_ncol[s]) * (long long)ld;
+          else if (row < it.rlim)
+            out = reinterpret_cast<T*>(a.Wp) + ((long long)tk.w * 64 + r) * ld;
+        } else if (it.c0 + r < it.clim) {
+          if (tk.w < 0)
+            out = reinterpret_cast<T*>(a.Wb) + a.c0 + (long long)(a.sn_first[s] + it.c0 + r) * ld;
+          else
+            out = reinterpret_cast<T*>(a.Wp) + ((long long)tk.w * 64 + r) * ld;
         }
-      } else if (it.c0 + r < it.clim) {
-        if (tk.w < 0) {
-          T* Wb = reinterpret_cast<T*>(a.Wb) + a.c0 + (long long)a.sn_first[s] * ld;
-          Wb[(long long)(it.c0 + r) * ld + c] = v;
-        } else {
-          T* part = reinterpret_cast<T*>(a.Wp) + (long long)tk.w * 64 * ld;
-          part[(long long)r * ld + c] = v;
-        }
+        if (out) out[h + c] = v;
       }
     }
+#pragma unroll
+    for (int c = 0; c < NR; ++c) acc[c] = F::zero();
   };
 #pragma unroll 1
   for (int u = 0; u < NST - 1; ++u) {
