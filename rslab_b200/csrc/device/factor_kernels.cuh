@@ -658,15 +658,8 @@ __global__ void __launch_bounds__(TPB) k_front_cb(FactorArgs fa, const int4* __r
 // Block reductions for the pivot search: max of a non-negative double with
 // the lowest index on ties (the reference's strict `>` scan).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void argmax_combine(double& v, int& i, double v2, int i2) {
-  if (v2 > v || (v2 == v && i2 < i)) {
-    v = v2;
-    i = i2;
-  }
-}
-
-// Warp-wide argmax_combine of every lane's (v, i), v >= 0 or -1 (none): the
-// same result (largest v, then smallest i) from three warp reductions on an
+// Warp-wide arg-max of every lane's (v, i), v >= 0 or -1 (none): largest v,
+// then smallest i, from three warp reductions on an
 // order-preserving key (bits of v + 1; 0 for none), instead of a shuffle tree.
 __device__ __forceinline__ void warp_argmax(double& v, int& i) {
   const unsigned long long key = v >= 0.0 ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
