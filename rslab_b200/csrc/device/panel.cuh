@@ -307,9 +307,11 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
   using Q = QuickTest<R>;
   const double alpha = (1.0 + sqrt(17.0)) / 8.0;
   // A quick test is only taken where the squares neither under- nor overflow,
-  // and above the static-pivot floor.
+  // and above the static-pivot floor (a floor past the range leaves no step to
+  // the quick test).
   const R a2m = (R)(alpha * alpha * (1.0 + (double)Q::margin));
-  const R lo2 = (R)fmax((double)Q::lo, pfloor > 0.0 ? fmin(pfloor * pfloor * (1.0 + (double)Q::margin), 1e38) : 0.0);
+  const double fl2 = pfloor > 0.0 ? pfloor * pfloor * (1.0 + (double)Q::margin) : 0.0;
+  const R lo2 = (R)fmin(fmax((double)Q::lo, fl2), 2.0 * (double)Q::hi);
   // x >= y for non-negative x, y: 1 / 0 where the margin decides it, -1 where
   // it does not (or a value may have under- or overflowed).
   auto quick_ge = [](double x, double y) -> int {

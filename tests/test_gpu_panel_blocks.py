@@ -8,6 +8,7 @@ import pytest
 
 from oracle.oracle import OracleSolver
 from rslab_b200 import CscMatrix, LdltSymbolic, Ordering, SolverSettings
+from rslab_b200.solver import ZeroPivotAction
 
 pytestmark = pytest.mark.gpu
 
@@ -40,6 +41,28 @@ def test_dense_panel_is_the_oracles(n, nb, dtype):
         assert np.array_equal(g.perm, o.perm)
         assert np.array_equal(g.d_diag, o.d_diag) and np.array_equal(g.d_subdiag, o.d_subdiag)
         assert np.array_equal(g.l_row_idx, o.l_row_idx) and np.array_equal(g.l_values, o.l_values)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128, np.float32, np.complex64])
+@pytest.mark.parametrize("engine", ["fma", "tensor"])
+def test_static_floor_above_1e19(dtype, engine):
+    """Every third pivot (5e19) lies below the floor of 1e20; the others (5e21) and the updates (1e16) leave no doubt."""
+    n = 40
+    a = dense_lower(n, dtype, False, 3)
+    v = a.values * dtype(1e18)
+    v[a.row_idx == np.repeat(np.arange(n), np.diff(a.col_ptr))] = np.where(np.arange(n) % 3 == 0, 5e19, 5e21)
+    a = CscMatrix(n, a.col_ptr, a.row_idx, v)
+    st = SolverSettings(ordering=Ordering.NATURAL, scaling="identity", schur_engine=engine,
+                        on_zero_pivot=ZeroPivotAction.perturb_to_eps(1e20))
+    sym = LdltSymbolic.analyze_with(a, st)
+    f = sym.factor(a, st)
+    o = OracleSolver(a, sym.export(), perturb_floor=1e20, scaling=False).factors()
+    assert f.n_perturbed() == o.n_perturbed == (n + 2) // 3
+    g = f.export_factors()
+    if engine == "fma":
+        assert np.array_equal(g.d_diag, o.d_diag) and np.array_equal(g.l_values, o.l_values)
+    else:  # at most 40 updates of a pivot, each rounded at its magnitude
+        assert np.max(np.abs(g.d_diag - o.d_diag) / np.abs(o.d_diag)) <= 40 * np.finfo(dtype).eps
 
 
 def test_wide_and_narrow_supernodes_of_one_level():
