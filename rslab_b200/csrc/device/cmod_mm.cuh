@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(MM_SPLIT_NT) k_split(FactorArgs fa, const int4
   constexpr bool CX = Field<T>::complex;
   constexpr int NOP = CX ? 6 : 4;  // A hi/lo, B hi/lo[, As, Bs]
   __shared__ __align__(16) float tile[NOP][MM_SPLIT_ROWS][MM_SPLIT_LD];
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   const int4 tk = tasks[blockIdx.x];
   const int k = tk.x, r0 = tk.y, ch = tk.z;
   const int first = fa.sn_first[k], ncol = fa.sn_ncol[k], nrow = fa.sn_nrow[k];
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(MM_NT, 1) k_cmod_mm(FactorArgs fa, const int4*
   using Sh = MmShape<T>;
   constexpr bool CX = Field<T>::complex;
   constexpr int NS = Sh::stages, NOP = Sh::nops, STAGE = mm_stage_bytes<T>();
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const uint32_t sraw = smem_u32(smem_raw);
   unsigned char* sm = smem_raw + (((sraw + 1023u) & ~1023u) - sraw);
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(ASM_NT, sizeof(T) >= 16 ? 1 : 2)
   __shared__ int2 spr[ASM_PB];      // (a, q0)
   __shared__ long long swb[ASM_PB];
   __shared__ int swl[ASM_PB];
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, r0 = (tk.y >> 16) * TC_M, c0 = (tk.y & 0xffff) * TC_N;
   const int ncol = fa.sn_ncol[s], nrow = fa.sn_nrow[s];
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(DM_NT) k_cmod_dmm(FactorArgs fa, const int4* _
   constexpr bool CX = Field<T>::complex;
   constexpr int KC = DmShape<T>::kc, DM_LDA = DmShape<T>::lda, DM_LDB = DmShape<T>::ldb;
   constexpr int STAGE = KC * (DM_LDA + DM_LDB);
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* stg = reinterpret_cast<T*>(smem_raw);
   const int4 tk = tasks[blockIdx.x];
@@ -800,7 +800,7 @@ __device__ __forceinline__ void dmm_lower_update(const T* A, const T* B, long lo
 template <typename T>
 __global__ void __launch_bounds__(DM_NT) k_schur_dmm(FactorArgs fa, const int4* __restrict__ tasks, int nb_small,
                                                     int nb_big) {
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* stg = reinterpret_cast<T*>(smem_raw);
   T* d_s = stg + 2 * DmShape<T>::kc * (DmShape<T>::lda + DmShape<T>::ldb);
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(DM_NT) k_schur_dmm(FactorArgs fa, const int4* 
 // lower part; D, dsub and kind read through ld_G from the factor's arrays.
 template <typename T>
 __global__ void __launch_bounds__(DM_NT) k_front_cb_dmm(FactorArgs fa, const int4* __restrict__ tasks) {
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* stg = reinterpret_cast<T*>(smem_raw);
   const int4 tk = tasks[blockIdx.x];

@@ -107,7 +107,7 @@ constexpr int MG_ROWS = 1024;
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_make_g(FactorArgs fa, const int4* __restrict__ tasks) {
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   const int4 tk = tasks[blockIdx.x];
   const int k = tk.x, t0 = tk.y, r0 = tk.z;
   const int first = fa.sn_first[k], ncol = fa.sn_ncol[k], nrow = fa.sn_nrow[k];
@@ -469,7 +469,7 @@ struct SchurSrc {
 template <typename T>
 __global__ void __launch_bounds__(TC_NT, 1) k_schur_tc(FactorArgs fa, const int4* __restrict__ tasks, int nb_small,
                                                        int nb_big) {
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];  // re-aligned to 1024 inside
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, kb = tk.y, r0 = tk.z, c0 = tk.w;

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(CM_NT, 2) k_cmod(FactorArgs fa, const int4* __
   using F = Field<T>;
   constexpr int KC = CmChunk<T>::v, NST = CmChunk<T>::stages;
   constexpr int STAGE = 2 * KC * TILE;  // A chunk [t][64 rows] then B chunk [t][64 cols]
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* acc_s = reinterpret_cast<T*>(smem_raw);  // [64 cols][64 rows]
   T* stg = acc_s + TILE * TILE;               // NST stages
@@ -510,7 +510,7 @@ template <typename T>
 __global__ void __launch_bounds__(TPB) k_schur(FactorArgs fa, const int4* __restrict__ tasks, int nb_small,
                                                int nb_big) {
   using F = Field<T>;
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* As = reinterpret_cast<T*>(smem_raw);
   T* Bs = As + KChunk<T>::v * TILE;
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(256) k_extend_add(FactorArgs fa, const int4* _
                                                     const int* __restrict__ emap,
                                                     const long long* __restrict__ emoff) {
   using F = Field<T>;
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, ncol = fa.sn_ncol[s], nrow = fa.sn_nrow[s], ms = nrow - ncol;
   T* panel = reinterpret_cast<T*>(fa.panel) + fa.sn_poff[s];
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(256) k_extend_add(FactorArgs fa, const int4* _
 template <typename T>
 __global__ void __launch_bounds__(TPB) k_front_cb(FactorArgs fa, const int4* __restrict__ tasks) {
   using F = Field<T>;
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* As = reinterpret_cast<T*>(smem_raw);
   T* Bs = As + KChunk<T>::v * TILE;
@@ -714,7 +714,7 @@ __global__ void k_force_floor(const unsigned long long* __restrict__ amax, doubl
 template <typename T>
 __global__ void k_drop_tol(FactorArgs fa, double tau) {
   using F = Field<T>;
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   const int s = blockIdx.x;
   const int first = fa.sn_first[s], ncol = fa.sn_ncol[s], nrow = fa.sn_nrow[s];
   T* panel = reinterpret_cast<T*>(fa.panel) + fa.sn_poff[s];

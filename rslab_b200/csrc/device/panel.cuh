@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
   using F = Field<T>;
   constexpr int NT = G * G, NW = NT / 32, PWM = G * NS, PWS = PWM + 1;
   constexpr int NE = NS * (NS + 1) / 2;
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   const double pfloor = fa.floor_dev ? *fa.floor_dev : fa.perturb_floor;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int4 tk = tasks[blockIdx.x];
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(DEEP_NT) k_deep(FactorArgs fa, const int4* __r
                                                   int nb_big) {
   using F = Field<T>;
   constexpr int PWM = 8 * NSL;
-  if (fa.status[0] != 0) return;
+  if (factor_failed(fa.status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int4 tk = tasks[blockIdx.x];
   const int s = tk.x, kb = tk.y, r0 = tk.w;

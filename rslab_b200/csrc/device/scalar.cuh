@@ -125,4 +125,13 @@ struct FieldC {
 template <> struct Field<c64> : FieldC<double> { using Lo = c32; };
 template <> struct Field<c32> : FieldC<float> { using Lo = c32; };
 
+// Whether the factorization has failed already, as one answer for the whole
+// CTA (every thread calls it).  A panel block that fails sets the word while
+// CTAs of its own launch and of the side streams start: warps that each read
+// it for themselves could disagree, and a CTA would run on without the warp
+// that initialises its shared words and barriers.
+__device__ __forceinline__ bool factor_failed(const int* status) {
+  return __syncthreads_or(*reinterpret_cast<const volatile int*>(status) != 0) != 0;
+}
+
 }  // namespace rsd

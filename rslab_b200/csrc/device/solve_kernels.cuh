@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(DI_NT) k_diag_inv(const int2* __restrict__ tas
                                                     const int* __restrict__ status, T* __restrict__ linv,
                                                     const long long* __restrict__ linv_off) {
   using F = Field<T>;
-  if (status[0] != 0) return;
+  if (factor_failed(status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls = reinterpret_cast<T*>(smem_raw);  // Ls[i * (TB + 1) + k] = L[i, k], k < i
   T* Xs = Ls + TB * (TB + 1);               // Xs[k * (TB + 1) + j] = X[k, j]
