@@ -295,9 +295,13 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     ds_s[i] = F::zero();
     d_s[i] = F::zero();
     kd_s[i] = 0;
-    if (reuse)
-      rec_s[i] = prec[i];
-    else if (prec)
+    if (reuse) {
+      // (a block that no factor has finished yet may have no record, or part
+      // of one: a step that reaches outside the block's remaining rows is
+      // taken in place)
+      const int code = prec[i], q = code < 0 ? -code - 1 : code;
+      rec_s[i] = q < pw && q >= i + (code < 0) ? code : i;
+    } else if (prec)
       prec[i] = i;  // a 1x1 step in place, unless slow_step records another
   }
   if (tid < 16) ctl[tid] = 0;

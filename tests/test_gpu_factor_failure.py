@@ -1,14 +1,16 @@
 """A factor that fails in one panel block while other blocks of the level and
 the side streams' kernels start: every CTA must take one decision (stop or go
 on), the call reports the rank deficiency, and the handle stays usable."""
+import ctypes as C
 import re
 from pathlib import Path
 
 import numpy as np
 import pytest
 
-from rslab_b200 import CscMatrix, LdltSymbolic, SolverSettings, matgen
-from rslab_b200.solver import NumericallyRankDeficient
+from rslab_b200 import CscMatrix, LdltSymbolic, Ordering, SolverSettings, matgen
+from rslab_b200 import _native as N
+from rslab_b200.solver import LdltSolver, NumericallyRankDeficient
 
 DEVICE = Path(__file__).resolve().parents[1] / "rslab_b200" / "csrc" / "device"
 
@@ -52,4 +54,29 @@ def test_failed_factor_of_many_blocks_leaves_the_handle_usable(engine, dtype):
     f.refactor(a)
     g = f.export_factors()
     for k in ("two_by_two", "perm", "d_diag", "d_subdiag", "l_values"):
+        assert np.array_equal(getattr(g, k), getattr(ref, k)), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [np.float64, np.complex64])
+def test_pivot_reuse_before_any_block_has_a_record(dtype):
+    """Pivot reuse on a handle whose only factor failed in its first block: the steps without a record are taken in
+    place, which on a dominant matrix is what the search chooses too."""
+    n = 193
+    rng = np.random.default_rng(1)
+    c, r = np.triu_indices(n)
+    v = rng.standard_normal(r.size).astype(dtype)
+    v[r == c] += 4 * n
+    a = CscMatrix.from_triplets(n, r, c, v)
+    st = SolverSettings(ordering=Ordering.NATURAL, scaling="identity", schur_engine="fma")
+    sym = LdltSymbolic.analyze_with(a, st)
+    ref = sym.factor(a, st).export_factors()
+    h, fs, zero = C.c_void_p(), st._factor_c(None), np.zeros_like(a.values)
+    code = {np.float64: N.F64, np.complex64: N.C32}[dtype]
+    assert N.lib.rslab_factor(sym._h, code, zero.ctypes.data_as(C.c_void_p), 0, C.byref(fs), C.byref(h)) != 0 and h
+    f = LdltSolver(h, sym, dtype)
+    f.reuse_pivots(True)
+    f.refactor(a)
+    g = f.export_factors()
+    for k in ("two_by_two", "perm", "d_diag", "l_values"):
         assert np.array_equal(getattr(g, k), getattr(ref, k)), k
