@@ -41,6 +41,7 @@
 // Reference: src/numeric/multifrontal_ldlt.rs:2400-3256.
 #pragma once
 
+#include <type_traits>
 #include <utility>
 
 #include "factor_kernels.cuh"
@@ -121,16 +122,38 @@ __device__ __forceinline__ cplx<R> panel_recip(cplx<R> a) {
   return Field<cplx<R>>::recip(a);
 }
 
+// u w, rounded at its own magnitude (one rounding in a component's first
+// product, one in the sum).
+template <typename T>
+__device__ __forceinline__ T product(T u, T w) {
+  if constexpr (Field<T>::complex)
+    return T{fma(-u.im, w.im, u.re * w.re), fma(u.re, w.im, u.im * w.re)};
+  else
+    return u * w;
+}
 // e - u w: the reference's multiply and subtract, each rounded (zero
-// multipliers skipped, as there), or fused.
+// multipliers skipped, as there), or fused.  The fused complex form rounds e
+// once: two fused operations in a row on e round it twice, which lost 1.3 to
+// 2.2 times the reference's accuracy on a dominant block.
 template <typename T, bool EXACT>
 __device__ __forceinline__ T minus_prod(T e, T u, T w) {
   using F = Field<T>;
   if constexpr (EXACT)
     return sel(F::is_zero(w), e, F::sub(e, F::mul(u, w)));
+  else if constexpr (F::complex)
+    return F::sub(e, product(u, w));
   else
     return F::fnma(u, w, e);
 }
+// Whether the updates of an entry are summed by themselves and subtracted from
+// it once, when its column is due, instead of one after another: the c32
+// instances of the tensor engine.  A sum of updates is smaller than the entry
+// of a dominant matrix and so are its roundings: residual of a 64-column block
+// a fifth, error of the refined 27-point sweep (24^3, lowest frequency) 5.8e-14
+// -> 5.1e-14, for 34.1 -> 34.7 ms a 64^3 factor.  The other fields reach the
+// accuracy of their sequential reference without it.
+template <typename T, bool EXACT>
+inline constexpr bool kSumUpdates = !EXACT && std::is_same_v<T, c32>;
 // 1 / a for the multipliers: the reference's two divisions of a complex
 // reciprocal, or one reciprocal of |a|^2.
 template <typename T, bool EXACT>
@@ -164,20 +187,27 @@ __device__ __forceinline__ void deep_rows(T* panel, long long nrow, int kb, int 
                                           const T* Lp, const int* src, const T* inv, const T* dd, const T* ds,
                                           const unsigned char* kd, bool any2) {
   using F = Field<T>;
+  constexpr bool SUM = kSumUpdates<T, EXACT>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int t = lane >> 2, r = lane & 3;
   for (int r0 = r_begin + 4 * warp; r0 < r_end; r0 += 4 * nw) {
     const int row = r0 + r;
     const bool live = row < r_end;
-    T x[NSL];
-#pragma unroll
-    for (int s = 0; s < NSL; ++s) {
+    auto entry = [&](int s) -> T {
       const int col = t + 8 * s;
-      x[s] = (live && col < pw) ? panel[row + (long long)(kb + src[col]) * nrow] : F::zero();
-    }
+      return (live && col < pw) ? panel[row + (long long)(kb + src[col]) * nrow] : F::zero();
+    };
+    T x[NSL];  // the row, or the sums of its updates until a slot's columns are due
+#pragma unroll
+    for (int s = 0; s < NSL; ++s) x[s] = SUM ? F::zero() : entry(s);
+    T due = SUM ? entry(0) : F::zero();
 #pragma unroll
     for (int s0 = 0; s0 < NSL; ++s0) {
       if (8 * s0 >= pw) break;
+      if constexpr (SUM) {
+        x[s0] = F::sub(due, x[s0]);
+        if (s0 + 1 < NSL) due = entry(s0 + 1);
+      }
       const int te = min(8, pw - 8 * s0);
       // (columns past pw read what follows in L's allocation and are not used)
 #pragma unroll 2
@@ -188,7 +218,7 @@ __device__ __forceinline__ void deep_rows(T* panel, long long nrow, int kb, int 
         for (int s = s0; s < NSL; ++s) {
           const T l0 = Lk[8 * s];
           const T l = s > s0 ? l0 : sel(t > t0, l0, F::zero());
-          x[s] = minus_prod<T, EXACT>(x[s], xk, l);
+          x[s] = SUM && s > s0 ? F::add(x[s], product(xk, l)) : minus_prod<T, EXACT>(x[s], xk, l);
         }
       }
     }
@@ -280,13 +310,20 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ty = tid % G, tx = tid / G;
   auto ix = [](int ii, int jj) constexpr { return jj * NS - jj * (jj - 1) / 2 + (ii - jj); };
+  // SUM: a[] holds the sum of an entry's updates, the entry itself waits in its
+  // place of the packed L, which only its thread reads or writes until its
+  // column is due
+  constexpr bool SUM = kSumUpdates<T, EXACT>;
   T a[NE];
 #pragma unroll
   for (int jj = 0; jj < NS; ++jj)
 #pragma unroll
     for (int ii = jj; ii < NS; ++ii) {
       const int i = ty + G * ii, j = tx + G * jj;
-      a[ix(ii, jj)] = (i < pw && i >= j) ? panel[(kb + i) + (long long)(kb + j) * nrow] : F::zero();
+      const bool in = i < pw && i >= j;
+      const T e = in ? panel[(kb + i) + (long long)(kb + j) * nrow] : F::zero();
+      a[ix(ii, jj)] = SUM ? F::zero() : e;
+      if (SUM && in) Lp[pk_col(j, pw) + i] = e;
     }
   if (kb == 0)
     for (int p = tid; p < ncol; p += NT) fa.lperm[first + p] = p;
@@ -340,15 +377,28 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
   // every step (a copy per slot column measured 1.3x slower: a block is
   // short, and each copy is fetched anew).
   int off = 0, nact = (pw + G - 1) / G;
+  // SUM: the entries of column c, which will be column cx of slot column 0
+  // (read ahead of the column's last update; in decide: 35.2 ms).
+  auto due_entries = [&](int c, int cx, T (&e)[NS]) __attribute__((always_inline)) {
+    const int lc = pk_col(c, pw);
+#pragma unroll
+    for (int ii = 0; ii < NS; ++ii) {
+      const int r = ty + G * ii - cx;
+      e[ii] = Lp[(tx == cx) & (r >= 0) & (r < pw - c) ? lc + c + r : npk];
+    }
+  };
   // The warp that owns column c: publish it (set `par`) with the multipliers
   // of a 1x1 pivot in place, which go straight into L.  Returns true in a lane
   // whose entries leave |a_cc| >= alpha max_i |a_ic| in doubt; such a step
   // (the block barrier collects the lanes' answers) is redone by slow_step.
   // Branch-free: lanes without a part in the column store into the padding.
-  auto decide = [&](int c, int par) __attribute__((always_inline)) -> bool {
+  auto decide = [&](int c, int par, const T (&e)[NS]) __attribute__((always_inline)) -> bool {
     T* u1 = pub + 2 * par * PWS;
     const int cx = c - off;
-    const T akk = shfl_t(a[0], (cx * G + cx) & 31);
+    T cv[NS];  // the column
+#pragma unroll
+    for (int ii = 0; ii < NS; ++ii) cv[ii] = SUM ? F::sub(e[ii], a[ix(ii, 0)]) : a[ix(ii, 0)];
+    const T akk = shfl_t(cv[0], (cx * G + cx) & 31);
     const R akk2 = quick2(akk);
     const T dinv = step_recip<T, EXACT>(akk);
     const int rem = pw - c, lc = pk_col(c, pw);
@@ -358,7 +408,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     for (int ii = 0; ii < NS; ++ii) {
       const int r = ty + G * ii - cx;  // row - c
       const bool mine = (tx == cx) & (r >= 0) & (r < rem);
-      const T col = a[ix(ii, 0)], w = F::mul(col, dinv);
+      const T col = cv[ii], w = F::mul(col, dinv);
       // true for NaN
       const bool big = !(quick2(col) * a2m <= akk2);
       doubt = doubt | (big & mine & (r != 0) & !reuse);
@@ -379,12 +429,14 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       for (int z = 1; z <= ii; ++z) c = sel(z == qs, a[ix(ii, z)], c);
 #pragma unroll
       for (int z = ii; z < NS - 1; ++z) r = sel(z == qs, a[ix(z, ii)], r);
-      if (ii < nact && tx == qx && (ii > qs || (ii == qs && ty >= tx))) v[off + ty + G * ii] = c;
-      if (ty == qx && (ii < qs || (ii == qs && tx < ty))) v[off + tx + G * ii] = r;
+      const int i = off + ty + G * ii, j = off + tx + G * ii;
+      if (ii < nact && tx == qx && (ii > qs || (ii == qs && ty >= tx)) && (!SUM || i < pw))
+        v[i] = SUM ? F::sub(Lp[pk_col(q, pw) + i], c) : c;
+      if (ty == qx && (ii < qs || (ii == qs && tx < ty))) v[j] = SUM ? F::sub(Lp[pk_col(j, pw) + q], r) : r;
     }
   };
-  // Row / column q of the registers := v.
-  auto read_col = [&](int q, const T* v) {
+  // Row / column q of the registers := v, from position p + 1 on.
+  auto read_col = [&](int q, const T* v, int p) {
     const int qs = (q - off) / G, qx = (q - off) % G;
 #pragma unroll
     for (int jj = 0; jj < NS; ++jj)
@@ -392,8 +444,16 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       for (int ii = jj; ii < NS; ++ii) {
         T e = a[ix(ii, jj)];
         const T vc = v[min(off + ty + G * ii, PWM - 1)], vr = v[min(off + tx + G * jj, PWM - 1)];
-        e = sel(tx == qx && jj == qs && (ii > jj || ty >= tx), vc, e);
-        a[ix(ii, jj)] = sel(ty == qx && ii == qs && (ii > jj || tx < ty), vr, e);
+        const bool inc = tx == qx && jj == qs && (ii > jj || ty >= tx);
+        const bool inr = ty == qx && ii == qs && (ii > jj || tx < ty);
+        if constexpr (SUM) {
+          const int i = off + ty + G * ii, j = off + tx + G * jj;
+          a[ix(ii, jj)] = sel(inc || inr, F::zero(), e);
+          if ((inc || inr) && i < pw && j > p) Lp[pk_col(j, pw) + i] = inr ? vr : vc;
+        } else {
+          e = sel(inc, vc, e);
+          a[ix(ii, jj)] = sel(inr, vr, e);
+        }
       }
   };
   // Step c by the reference's expressions: warp 0 tests the published column;
@@ -478,7 +538,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
 #pragma unroll
         for (int z = 0; z < NZ; ++z) {
           const int i = c + lane + 32 * z;
-          const double m = F::mag2(v2[min(i, pw - 1)]);
+          const double m = F::mag2(i == c ? u1[q] : v2[min(i, pw - 1)]);  // (column c is published, not written out)
           if ((i < pw) & (i != q) & (m > rmx)) rmx = m;
         }
         warp_argmax(rmx, idx);
@@ -579,7 +639,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     __syncthreads();
     const int kstep = ctl[4], p = ctl[5], kp = ctl[7];
     if (kp != p) {
-      read_col(kp, rep);
+      read_col(kp, rep, p);
       // rows p, kp of the finished columns (one warp throughout, so the
       // interchanges stay ordered)
       if (warp == NW - 1)
@@ -593,6 +653,8 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     return kstep;
   };
 
+  // One step's update of an entry (of its sum).
+  auto step_update = [](T e, T u, T w) -> T { return SUM ? F::fma_(u, w, e) : minus_prod<T, EXACT>(e, u, w); };
   bool failed = false;
   auto shift = [&]() __attribute__((always_inline)) {
 #pragma unroll
@@ -622,8 +684,8 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
           for (int jj = 0; jj < NS; ++jj)
             if (jj <= ii) {
               const T e = a[ix(ii, jj)], w = w1[off + tx + G * jj], wb = w2[off + tx + G * jj];
-              const T vb = EXACT ? F::sub(F::sub(e, F::mul(x, w)), F::mul(x2, wb)) : F::fnma(x2, wb, F::fnma(x, w, e));
-              const T v = minus_prod<T, EXACT>(e, x, w);
+              const T v = step_update(e, x, w);
+              const T vb = EXACT ? F::sub(F::sub(e, F::mul(x, w)), F::mul(x2, wb)) : step_update(v, x2, wb);
               a[ix(ii, jj)] = sel(kstep == 2, vb, v);
             }
         }
@@ -631,7 +693,11 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
     if (kn >= pw) break;
     if (kn - off >= G) shift();
     bool doubt = false;
-    if (warp == ((kn - off) * G) >> 5) doubt = decide(kn, par ^ 1);
+    T due[NS] = {};
+    if (warp == ((kn - off) * G) >> 5) {
+      if constexpr (SUM) due_entries(kn, kn - off, due);
+      doubt = decide(kn, par ^ 1, due);
+    }
     par ^= 1;
     k = kn;
     // runs of 1x1 pivots in place
@@ -642,6 +708,11 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       // update entries that nothing reads)
       const T* u1 = pub + 2 * par * PWS + off + ty;
       const T* w1 = Lp + pk_col(k - 1, pw) + off + tx;
+      const bool bnd = k - off == G;  // slot column 0 is finished
+      const int cx = bnd ? 0 : k - off;
+      const bool owner = warp == (cx * G) >> 5;
+      if constexpr (SUM)
+        if (owner) due_entries(k, cx, due);
       T ur[NS], wc[NS];
 #pragma unroll
       for (int ii = 0; ii < NS; ++ii) {
@@ -649,7 +720,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
         wc[ii] = w1[G * ii];
       }
       auto upd = [&](int ii, int jj) __attribute__((always_inline)) {
-        a[ix(ii, jj)] = minus_prod<T, EXACT>(a[ix(ii, jj)], ur[ii], wc[jj]);
+        a[ix(ii, jj)] = step_update(a[ix(ii, jj)], ur[ii], wc[jj]);
       };
       // the columns beyond slot column 0 (rows past the block are skipped
       // where that saves more than the branch)
@@ -665,13 +736,12 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
 #pragma unroll
       for (int ii = 0; ii < NS; ++ii) upd(ii, 0);
       par ^= 1;
-      const bool bnd = k - off == G;  // slot column 0 is finished
       if (bnd) {
         upd_rest();
         shift();
       }
       doubt = false;
-      if (warp == ((k - off) * G) >> 5) doubt = decide(k, par);
+      if (owner) doubt = decide(k, par, due);
       if (!bnd) upd_rest();
       slow = __syncthreads_or(doubt) != 0;
     }
