@@ -63,22 +63,32 @@ constexpr int CH_GROUPS = RHS_MAX / CH_NR;
 // blocks in a level from which its chains take every column of a pass
 constexpr int CH_WIDE_ITEMS = 600;
 
-// Stages: 4, three for 16-byte elements, two for 16 columns of the smaller ones
-// (the next unit loads while one is multiplied).
+// CTAs per SM of the streamed kernel, and with them its stages and the columns
+// whose slice partials are exchanged at a time.  Instances of one and four
+// columns: three CTAs, four stages (three for 16-byte elements).  Sixteen
+// columns in the single-precision fields: two stages (the next unit loads while one is
+// multiplied) and partials by halves, so that three CTAs fit instead of two
+// (64^3 mixed step 54.9 -> 52.6 ms; f32, 40 columns on 37 x 40 x 33: 3.53 ->
+// 3.39).  In double precision that costs more than it gives: f64 has three
+// stages and whole partials on two CTAs (40 columns on 24 x 25 x 23: 1.49 ms
+// with three CTAs and more spills, 1.44 so; on 150 x 140 1.13 and 1.07), c64
+// the same on one (two: 0.7% slower).
+template <typename T>
+__host__ __device__ constexpr bool st_three(int nr) {
+  return nr < 16 || sizeof(typename Field<T>::Real) == 4;
+}
 template <typename T>
 __host__ __device__ constexpr int st_stages(int nr) {
-  return sizeof(T) >= 16 ? 3 : nr >= 16 ? 2 : 4;
+  return nr >= 16 && st_three<T>(nr) ? 2 : nr >= 16 || sizeof(T) >= 16 ? 3 : 4;
 }
-// Columns whose slice partials are exchanged at a time, and the CTAs per SM the
-// kernel is compiled for.  Sixteen columns of 4- and 8-byte elements: two
-// stages and partials by halves, three CTAs per SM instead of two (64^3 mixed
-// step 54.9 -> 52.6 ms).  The same for c64 (two CTAs instead of one, 128
-// registers) was 0.7% slower, so c64 keeps one.
 template <typename T>
 __host__ __device__ constexpr int st_red_cols(int nr) {
-  return nr < 16 || sizeof(T) >= 16 ? nr : 8;
+  return nr >= 16 && st_three<T>(nr) ? 8 : nr;
 }
-__host__ __device__ constexpr int st_minb(size_t es, int nr) { return nr < 16 ? 3 : es >= 16 ? 1 : 3; }
+template <typename T>
+__host__ __device__ constexpr int st_minb(int nr) {
+  return st_three<T>(nr) ? 3 : sizeof(T) >= 16 ? 1 : 2;
+}
 
 // Right-hand-side buffers are sized by the pass's column count nr (<=
 // RHS_MAX), so a one-column solve keeps several CTAs resident per SM; the
@@ -274,7 +284,7 @@ __device__ __forceinline__ void st_issue(T* S, T* Vs, const StItem<T, FWD>& it, 
 }
 
 template <typename T, bool FWD, int NR>
-__global__ void __launch_bounds__(WV_NT, st_minb(sizeof(T), NR)) k_stream(SolveArgs a, const int4* __restrict__ tasks) {
+__global__ void __launch_bounds__(WV_NT, st_minb<T>(NR)) k_stream(SolveArgs a, const int4* __restrict__ tasks) {
   using F = Field<T>;
   constexpr int NST = st_stages<T>(NR), RC = st_red_cols<T>(NR);
   extern __shared__ __align__(16) unsigned char smem_raw[];
