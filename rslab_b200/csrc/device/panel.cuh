@@ -154,7 +154,9 @@ __device__ __forceinline__ T minus_prod(T e, T u, T w) {
 // accuracy of their sequential reference without it.
 template <typename T, bool EXACT>
 inline constexpr bool kSumUpdates = !EXACT && std::is_same_v<T, c32>;
-// 1 / a for the multipliers: the reference's two divisions of a complex
+// 1 / a for the multipliers of every 1x1 step, whichever path decides it (a
+// replay takes a recorded step in place on the quick path even where the
+// search needed the row maximum): the reference's two divisions of a complex
 // reciprocal, or one reciprocal of |a|^2.
 template <typename T, bool EXACT>
 __device__ __forceinline__ T step_recip(T a) {
@@ -509,7 +511,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       if (accept) {
         T dk = akk;
         if (!err) err = !perturb1(dk, lane == 0);
-        const T dinv = panel_recip(dk);
+        const T dinv = step_recip<T, EXACT>(dk);
         for (int i = c + 1 + lane; i < pw; i += 32) w1[i] = F::mul(u1[i], dinv);
         if (lane == 0) w1[c] = dk;
       }
@@ -561,7 +563,7 @@ __global__ void __launch_bounds__(G * G, getf2_minb(G, NS, sizeof(T)))
       if (kstep == 1) {
         T dk = kp == c ? v1c : v2q;
         err = !perturb1(dk, lane == 0);
-        const T dinv = panel_recip(dk);
+        const T dinv = step_recip<T, EXACT>(dk);
 #pragma unroll
         for (int z = 0; z < NZ; ++z) {
           const int i = c + 1 + lane + 32 * z;

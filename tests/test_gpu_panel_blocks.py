@@ -59,6 +59,22 @@ def ldl_residual(a, f, cols=None):
     return np.linalg.norm((A - L @ D @ L.T)[at]), np.linalg.norm((np.abs(L) @ np.abs(D) @ np.abs(L).T)[at])
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128, np.float32, np.complex64])
+@pytest.mark.parametrize("engine", ["fma", "tensor"])
+@pytest.mark.parametrize("n,nb", [(33, 64), (65, 64), (193, 64), (200, 128), (640, 64)])
+def test_replayed_interchanges_and_2x2_steps(n, nb, engine, dtype):
+    a = dense_lower(n, dtype, False, n)
+    st = SolverSettings(ordering=Ordering.NATURAL, panel_nb=nb, schur_engine=engine)
+    f = LdltSymbolic.analyze_with(a, st).factor(a, st)
+    g = f.export_factors()
+    assert g.two_by_two.any() and not np.array_equal(g.perm, np.arange(n))
+    f.reuse_pivots(True)
+    f.refactor(a)
+    h = f.export_factors()
+    for k in ("two_by_two", "perm", "d_diag", "d_subdiag", "l_values"):
+        assert np.array_equal(getattr(g, k), getattr(h, k)), k
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.complex64, np.complex128])
 @pytest.mark.parametrize("width,deep", [(33, 0), (64, 0), (128, 0), (64, 40), (64, 200)])
 def test_fused_panel_rounds_no_more_than_the_reference(width, deep, dtype):
