@@ -24,7 +24,6 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "-Xcompiler", "-ffp-contract=off",
     "--expt-relaxed-constexpr",
-    "-split-compile=0",  # device optimisation and assembly of a file's kernels on all host threads
 ]
 
 

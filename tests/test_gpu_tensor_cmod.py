@@ -108,10 +108,10 @@ def test_tensor_cmod_deterministic():
 
 @pytest.mark.parametrize("nb", [32, 64])
 def test_tensor_engine_with_panel_widths(nb):
-    """The tensor engine's panel kernels (left-looking getf2, block transform
-    of the deep rows, tensor-core in-panel Schur) with 32- and 64-wide blocks
-    (128 for the wide separators): on a fixed pivot sequence the factor
-    agrees with the FP64 one at fp32 level."""
+    """The tensor engine's panel kernels (fused getf2, deep rows, tensor-core
+    in-panel Schur) with 32- and 64-wide blocks (128 for the wide separators):
+    on a fixed pivot sequence the factor agrees with the FP64 one at fp32
+    level."""
     from rslab_b200 import Ordering
     a = spd3d(24, True)
     st = SolverSettings(ordering=Ordering.METIS_ND, panel_nb=nb)
