@@ -59,6 +59,22 @@ def ldl_residual(a, f, cols=None):
     return np.linalg.norm((A - L @ D @ L.T)[at]), np.linalg.norm((np.abs(L) @ np.abs(D) @ np.abs(L).T)[at])
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64, np.complex128])
+@pytest.mark.parametrize("n,nb", [(1, 64), (31, 64), (32, 64), (33, 64), (63, 64), (64, 64), (65, 64), (128, 64), (129, 64),
+                                  (193, 64), (150, 17), (200, 128), (513, 64), (600, 8), (640, 64)])
+def test_fused_panels_at_their_edges(n, nb, dtype):
+    """The tensor engine's instances (fused updates; pivots may differ from the oracle's): the factorization's
+    backward error |P A P^T - L D L^T| against its bound n u |L| |D| |L^T|, with 2 sqrt(n) for n (rounding errors
+    of random signs)."""
+    for dominant in (False, True):
+        a = dense_lower(n, dtype, dominant, n + nb)
+        st = SolverSettings(ordering=Ordering.NATURAL, scaling="identity", panel_nb=nb, schur_engine="tensor")
+        f = LdltSymbolic.analyze_with(a, st).factor(a, st).export_factors()
+        assert np.array_equal(np.sort(f.perm), np.arange(n))
+        r, s = ldl_residual(a, f)
+        assert r <= 2.0 * np.sqrt(n) * np.finfo(dtype).eps / 2 * s
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.complex128, np.float32, np.complex64])
 @pytest.mark.parametrize("engine", ["fma", "tensor"])
 @pytest.mark.parametrize("n,nb", [(33, 64), (65, 64), (193, 64), (200, 128), (640, 64)])
