@@ -294,10 +294,10 @@ int rslab_solve_profile(rslab_fac_handle* fac, int64_t nrhs, double* kind_ms, in
  * block-chain solve, 23 forward push partial-sum reduction, 24 multifrontal
  * contribution block, -1 other; 12, 16, 20, 21 and 22 are not launched any
  * more: the chain items gather their own right-hand sides and sum split dots,
- * and the deep rows need no block transform), grid size and device ms.  *count = rows available; at most cap are written.
- * A measurement aid with no reference counterpart.  Kinds 8-11 are the
- * tensor-core cmod's GEMM tiles, its assembly and the real / complex operand
- * split. */
+ * and the deep rows need no block transform), grid size and device ms.
+ * *count = rows available; at most cap are written.  A measurement aid with no
+ * reference counterpart.  Kinds 8-11 are the tensor-core cmod's GEMM tiles, its
+ * assembly and the real / complex operand split. */
 int rslab_profile_trace(const rslab_fac_handle* fac, int64_t cap, int32_t* kind, int32_t* grid, float* ms,
                         int64_t* count);
 /* Reference LdltFactors layout; pass NULL arrays to query *nnz_out first. */

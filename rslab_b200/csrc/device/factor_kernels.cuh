@@ -3,8 +3,8 @@
 // Data layout in HBM (one pool per factor handle, offsets fixed at analysis):
 //   panel[s]  : nrow_s x ncol_s column-major (stride nrow_s) at poff[s]; after
 //               the factor rows/cols are in the panel's pivot order, the
-//               strictly-lower part holds L (2x2 coupling entry = d21, never
-//               read as L), the diagonal holds D.
+//               strictly-lower part holds L (zero at a 2x2's coupling entry,
+//               whose d21 is in dsub), the diagonal holds D.
 //   e-indexed : d[n], dsub[n], kind[n] (0 = 1x1, 1/2 = first/second column of
 //               a 2x2 block), lperm[n] (pivot position -> pre-pivot local
 //               column) — e = first_col(s) + pivot position.
@@ -28,7 +28,10 @@ constexpr int TPB = 256;      // threads per CTA of the GEMM-class kernels
 // Deep rows that getf2 solves itself, for blocks of at most FUSE_PW columns:
 // two passes of its eight warps (10 us) against a launch of k_deep (about 8 us
 // with the launch); 192 rows took six.  A pass over 128 columns takes 45 us
-// (c32), so wider blocks always leave them to k_deep.
+// (c32), so wider blocks always leave them to k_deep.  On the two warps of the
+// narrow instance the same rows are eight passes (32 columns, f64: 14 to 18
+// us), which counts only where its launch has few blocks; launches that fill
+// the GPU with narrow blocks save the second reading of L.
 constexpr int FUSE_DEEP_ROWS = 64, FUSE_PW = 64;
 constexpr int EA_ROWS = 1024;        // front rows per extend-add task
 struct FactorArgs {

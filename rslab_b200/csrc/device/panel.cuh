@@ -23,13 +23,15 @@
 // sees the operations of the reference in its order, so with EXACT (the FMA
 // engine) the factor is the oracle's bit for bit in every field; the tensor
 // engine, whose products are summed in tiles anyway, takes fused updates and
-// one division per complex reciprocal, except in real f64 (64-column block
-// with either form: c32 44 / 32 us, 128 columns of c64 104 / 75, f64 31 / 28).
-// The finished columns collect in shared memory (packed lower triangle).
-// Measured (B200): a diagonally dominant 64-column block on one CTA takes 31
-// us in f64 and 42 us in c32 (0.35 and 0.5 us a step); a shared-memory block
-// with per-step trailing updates took 2.4 us a step.  All panel launches of a
-// refactor: 128^2 f64 4.65 -> 2.02 ms, 64^3 c32 20.3 -> 11.5 ms.
+// one division per complex reciprocal, except in real f64 (see minus_prod and
+// kSumUpdates for how its updates round).  The finished columns collect in
+// shared memory (packed lower triangle).
+// Measured (B200), a diagonally dominant block on one CTA, FMA engine / fused:
+// 64 columns of f64 31 / 27 us, f32 28 / 25, c64 61 / 41, c32 43 / 35; 128
+// columns of f64 49 / 41, f32 40 / 35, c64 111 / 80, c32 62 / 52 (0.4 to 0.7 us
+// a step; an indefinite block of random entries twice that).  A shared-memory
+// block with per-step trailing updates took 2.4 us a step.  All panel launches
+// of a refactor: 128^2 f64 4.65 -> 1.70 ms, 64^3 c32 20.3 -> 10.1 ms.
 //
 // k_deep.  The interchanges of a block permute its columns before any step
 // touches a deep row, so the replay is X = (X P) L^-T D^-1 with the final L:
@@ -37,7 +39,7 @@
 // 8 s in slot s); a step is one shuffle of x_k and one multiply-subtract per
 // later slot, L read from shared memory.  Bound by that chain (64 steps); it
 // needs no separate block transform: deep rows of a 64^3 c32 refactor 11.1 ->
-// 5.5 ms in 169 launches instead of 334.
+// 5.6 ms in 169 launches instead of 334.
 // Reference: src/numeric/multifrontal_ldlt.rs:2400-3256.
 #pragma once
 

@@ -54,7 +54,7 @@ struct SolveArgs {
   const int2* dots_red;   // per supernode: (first partial-sum slot, row chunks) of its split backward dots
   const void* linv;       // inverses of the TB x TB diagonal blocks of wide supernodes
   const long long* linv_off;
-  void* Wp;               // slots x 32 x ld partial sums of the split backward dots
+  void* Wp;               // slots x 64 x ld partial sums of the split pushes and backward dots
   int* wstate;            // chain solves: status, abort word, ticket counters
   int ld;     // row stride (total rhs count)
   int c0;     // first rhs column of this pass

@@ -52,8 +52,8 @@ constexpr long WV_POLL_LIMIT = 1L << 21;  // polls before a wait gives up
 constexpr int ST_UNIT = 2112;             // streamed tile elements (max of 32 x 65 and 64 x 33)
 constexpr int CH_UNIT = 64 * 65;          // chain tile elements
 // Units (32 x 64 panel tiles) that a streamed item takes one after another: a
-// level's units over ST_ITEMS items (two CTAs per SM, twice), within these
-// bounds.  Fixed items of 16 units left the upper levels with 20 to 300 items
+// level's units over ST_ITEMS items (four per SM: the kernel runs one to three
+// CTAs on an SM, see st_minb), within these bounds.  Fixed items of 16 units left the upper levels with 20 to 300 items
 // of 30 to 50 us each.
 constexpr int ST_ITEMS = 4 * 148, ST_UNITS_MIN = 2, ST_UNITS_MAX = 16;
 // The right-hand sides of a pass are solved as CH_GROUPS independent chains
@@ -105,7 +105,7 @@ __host__ __device__ constexpr size_t st_smem_bytes(int nr) {
   return ((size_t)st_stages<T>(nr) * st_stage_elems<T>(nr) + 4 * 65 * st_red_cols<T>(nr)) * sizeof(T) + 16;
 }
 // Chain: one tile slot (its copy overlaps the wait for the dependency's
-// flag; after the chain it holds the slice partials), the inverse block,
+// values; after the chain it holds the slice partials), the inverse block,
 // right-hand sides (64 x nr) and the block vector (64 x nr).
 template <typename T>
 __host__ __device__ constexpr size_t ch_smem_bytes(int nr) {

@@ -1371,8 +1371,8 @@ void enqueue_factor(rslab_fac_handle& F, Prof* prof = nullptr) {
       case L_GETF2:
         // the FMA engine in the oracle's operation order, the tensor engine
         // fused, except real f64: a near-singular KKT fixture flips the sign of
-        // a pivot with fused updates (which would save 10% there, against 20-30%
-        // in the complex fields)
+        // a pivot with fused updates (which would save 13% there, against a
+        // third in c64 and a fifth in c32)
         if (mm)
           launch_getf2<T, std::is_same_v<T, double>>(L.nb_slot, L.ntasks, ls, fa, H.d_t4 + L.task_off, nb_small, nb_big);
         else
@@ -2846,7 +2846,10 @@ namespace {
 constexpr int64_t NOALLOC_MAX_NROW = 4096;
 constexpr int64_t NOALLOC_MAX_NCOL = 1024;
 constexpr size_t NOALLOC_BYTES = size_t(1) << 20;
-constexpr int NOALLOC_FUSE_ROWS = 192;  // deep rows that a block's getf2 solves itself (fewer task-list entries)
+// Deep rows that a block's getf2 solves itself: their chunks need no entries in
+// the task list, which counts towards the scratch limit (in time, 192 rows under
+// 32 columns take 86 us this way and 256 rows 40 us by k_deep).
+constexpr int NOALLOC_FUSE_ROWS = 192;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
